@@ -659,9 +659,10 @@ __global__ void k_collapse4(const BvhNode* __restrict__ bin, uint32_t first, uin
   int32_t oc[4], on[4];
   for (int j = 0; j < 4; ++j) {
     const bool used = j < k;
-    ox[j] = used ? lo[j][0] : 0.0f; oX[j] = used ? hi[j][0] : 0.0f;
-    oy[j] = used ? lo[j][1] : 0.0f; oY[j] = used ? hi[j][1] : 0.0f;
-    oz[j] = used ? lo[j][2] : 0.0f; oZ[j] = used ? hi[j][2] : 0.0f;
+    // An absent child's box is inside out, so that no ray enters it.
+    ox[j] = used ? lo[j][0] : kFloatMax; oX[j] = used ? hi[j][0] : -kFloatMax;
+    oy[j] = used ? lo[j][1] : kFloatMax; oY[j] = used ? hi[j][1] : -kFloatMax;
+    oz[j] = used ? lo[j][2] : kFloatMax; oZ[j] = used ? hi[j][2] : -kFloatMax;
     oc[j] = used ? ref[j] : kEmptyChild;
     on[j] = used ? cnt[j] : 0;
     if (used && ref[j] < 0 && !leaves_are_instances) {
@@ -671,13 +672,15 @@ __global__ void k_collapse4(const BvhNode* __restrict__ bin, uint32_t first, uin
       oc[j] = (int32_t)~((first << kLeafCountBits) | (count - 1u));
     }
   }
-  Bvh4Node w;
-  w.lo_x = make_float4(ox[0], ox[1], ox[2], ox[3]); w.hi_x = make_float4(oX[0], oX[1], oX[2], oX[3]);
-  w.lo_y = make_float4(oy[0], oy[1], oy[2], oy[3]); w.hi_y = make_float4(oY[0], oY[1], oY[2], oY[3]);
-  w.lo_z = make_float4(oz[0], oz[1], oz[2], oz[3]); w.hi_z = make_float4(oZ[0], oZ[1], oZ[2], oZ[3]);
-  w.child = make_int4(oc[0], oc[1], oc[2], oc[3]);
-  w.count = make_int4(on[0], on[1], on[2], on[3]);
-  wide[i] = w;
+  float4* rows = reinterpret_cast<float4*>(wide + i);
+  rows[node_row(i, 0)] = make_float4(ox[0], ox[1], ox[2], ox[3]);
+  rows[node_row(i, 1)] = make_float4(oX[0], oX[1], oX[2], oX[3]);
+  rows[node_row(i, 2)] = make_float4(oy[0], oy[1], oy[2], oy[3]);
+  rows[node_row(i, 3)] = make_float4(oY[0], oY[1], oY[2], oY[3]);
+  rows[node_row(i, 4)] = make_float4(oz[0], oz[1], oz[2], oz[3]);
+  rows[node_row(i, 5)] = make_float4(oZ[0], oZ[1], oZ[2], oZ[3]);
+  reinterpret_cast<int4*>(rows)[node_row(i, 6)] = make_int4(oc[0], oc[1], oc[2], oc[3]);
+  reinterpret_cast<int4*>(rows)[node_row(i, 7)] = make_int4(on[0], on[1], on[2], on[3]);
 }
 
 // Refit after a point edit (the reference refits its BLAS there,

@@ -671,11 +671,12 @@ __global__ void k_cache_base(CacheQueues C, PathState P) {
 
 constexpr unsigned kFullWarp = 0xFFFFFFFFu;
 // Resident blocks per SM the persistent tracing kernels are compiled for:
-// seven blocks of 128 (72 registers a thread; the extension walk spills a
-// few words to L1) hide more of the node loads' latency than six at 80
-// registers (sphere field, 1080p: extension kernels 2.30 -> 2.16 ms per
-// sample together with the approximate slab reciprocal and the evict_last
-// node loads).
+// seven blocks of 128 (72 registers a thread, no spills in the plain
+// instantiations now that the world ray, the closest hit and the path's slot
+// and random state wait in shared memory, SharedStore). At eight (64
+// registers) the extension kernel spills 32 bytes a thread: 16 rooms of a
+// batch 41.2 -> 39.1 ms and the sphere field 11.73 -> 11.65, but the box room
+// 1.84 -> 1.99, textured scenes 0.60 -> 0.68 and glTF 0.47 -> 0.49.
 constexpr int kTraceBlocksPerSm = 7;
 constexpr uint32_t kDefaultRefillBelow = 24;
 
@@ -709,6 +710,8 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_shadow(SceneVi
   uint32_t rays = 0;
   Walk W;
   WalkStack stack;
+  __shared__ SharedStore<kBlock>::Block held;
+  SharedStore<kBlock> store{held};
   uint32_t rng = 0;
   uint32_t index = 0, scene = 0;
   bool active = false, exhausted = false;
@@ -719,12 +722,12 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_shadow(SceneVi
       if (kBatch) scene = table_scene(B, __float_as_uint(Q.shadow.thr[index].w));
       const float4 ro = Q.shadow.ray_o[index];
       const float4 rd = Q.shadow.ray_d[index];
-      walk_begin(kBatch ? B.views[scene] : S, W, V(ro), V(rd), 0.0f, ro.w);
+      walk_begin(kBatch ? B.views[scene] : S, W, store, V(ro), V(rd), 0.0f, ro.w);
       active = true;
       ++rays;
     }
     if (!__any_sync(kFullWarp, active)) break;
-    if (walk_round<true, kCount, kFullShading>(kBatch ? B.views[scene] : S, W, stack, rng, active, &vc)) {
+    if (walk_round<true, kCount, kFullShading>(kBatch ? B.views[scene] : S, W, store, stack, rng, active, &vc)) {
       active = false;
       const float tr = W.transmittance;
       if (tr > 0.0f) {
@@ -812,12 +815,15 @@ __global__ void k_fill_float(float* __restrict__ out, uint32_t n, float value) {
 
 // The ReSTIR passes' queued visibility rays (VisibilityQueue), as a
 // persistent any-hit kernel that completes each ray's pixel record.
+template <bool kFullShading>
 __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_visibility(SceneView S, VisibilityQueue VQ,
     uint32_t pass, unsigned char* __restrict__ records, uint32_t stride, uint32_t positive,
     uint32_t refill_below) {
   const uint32_t n = VQ.counters[2 * pass];
   Walk W;
   WalkStack stack;
+  __shared__ SharedStore<kBlock>::Block held;
+  SharedStore<kBlock> store{held};
   uint32_t rng = 0, index = 0;
   bool active = false, exhausted = false;
   for (;;) {
@@ -825,11 +831,11 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_visibility(SceneV
     if (got < n) {
       index = got;
       const float4 o = VQ.origin[index];
-      walk_begin(S, W, V(o), V(VQ.direction[index]), 0.0f, o.w);
+      walk_begin(S, W, store, V(o), V(VQ.direction[index]), 0.0f, o.w);
       active = true;
     }
     if (!__any_sync(kFullWarp, active)) break;
-    if (walk_round<true, false>(S, W, stack, rng, active, nullptr)) {
+    if (walk_round<true, false, kFullShading>(S, W, store, stack, rng, active, nullptr)) {
       active = false;
       const float visibility = W.transmittance;
       const uint32_t slot = VQ.slot[index];
@@ -863,27 +869,34 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_extend(SceneVi
   uint32_t rays = 0;
   Walk W;
   WalkStack stack;
-  uint32_t rng = 0, rng0 = 0, slot = 0, scene = 0;
+  __shared__ SharedStore<kBlock>::Block held;
+  SharedStore<kBlock> store{held};
+  // The path's slot and random state (only coverage tests draw from it), in
+  // shared memory too.
+  __shared__ uint32_t held_slot[kBlock], held_rng[kBlock], held_rng0[kBlock];
+  uint32_t &slot = held_slot[threadIdx.x], &rng = held_rng[threadIdx.x], &rng0 = held_rng0[threadIdx.x];
+  uint32_t scene = 0;
   bool active = false, exhausted = false;
   for (;;) {
     const uint32_t got = warp_fetch(fetch, n, active, refill_below, exhausted);
     if (got < n) {
-      slot = rays_in[got];
-      if (kBatch) scene = table_scene(B, slot);
-      const float4 o = P.origin[slot];
-      const float4 d = P.direction[slot];
-      rng = rng0 = __float_as_uint(P.radiance[slot].w);
-      walk_begin(kBatch ? B.views[scene] : S, W, V(o), V(d), o.w, d.w);
+      const uint32_t at = rays_in[got];
+      slot = at;
+      if (kBatch) scene = table_scene(B, at);
+      const float4 o = P.origin[at];
+      const float4 d = P.direction[at];
+      rng = rng0 = __float_as_uint(P.radiance[at].w);
+      walk_begin(kBatch ? B.views[scene] : S, W, store, V(o), V(d), 0.0f, d.w);
       active = true;
       ++rays;
     }
     if (!__any_sync(kFullWarp, active)) break;
     bool emit = false;
     const SceneView& SS = kBatch ? B.views[scene] : S;
-    if (walk_round<false, kCount, kFullShading>(SS, W, stack, rng, active, &vc)) {
+    if (walk_round<false, kCount, kFullShading>(SS, W, store, stack, rng, active, &vc)) {
       active = false;
-      if (W.found) {
-        P.hit[slot] = make_uint4(W.best_instance, W.best_tri, __float_as_uint(W.b1), __float_as_uint(W.b2));
+      if (W.is(kWalkFound)) {
+        P.hit[slot] = store.hit();
         if (rng != rng0) P.radiance[slot].w = __uint_as_float(rng);
         emit = true;
       } else {
@@ -891,7 +904,7 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_extend(SceneVi
         const float4 thr = P.throughput[slot];
         const uint32_t flags = thr.w < 0.0f ? kUnweightedLight : 0u;
         const FrameConst& f = kBatch ? B.frames[scene] : *fcp;
-        const F3 R = miss_path<kAnalytic>(SS, f, W.origin, W.direction, flags, thr.w, V(thr), V(rad));
+        const F3 R = miss_path<kAnalytic>(SS, f, store.origin(), store.direction(), flags, thr.w, V(thr), V(rad));
         P.radiance[slot] = F4(R, 1.0f);
       }
     }
@@ -1517,8 +1530,9 @@ void launch_wavefront_batch(const SceneTable& B, uint32_t max_bounces, const Pat
 void launch_visibility(const SceneView& S, const VisibilityQueue& queue, uint32_t pass, unsigned char* records,
     uint32_t stride, bool positive, cudaStream_t stream, const TraceTuning& tuning) {
   const uint32_t refill = tuning.refill_below ? std::min(tuning.refill_below, 32u) : kDefaultRefillBelow;
-  const uint32_t grid = persistent_grid((const void*)k_visibility, queue.capacity, tuning);
-  k_visibility<<<grid, kBlock, 0, stream>>>(S, queue, pass, records, stride, positive ? 1u : 0u, refill);
+  const auto kernel = S.full_shading != 0 ? k_visibility<true> : k_visibility<false>;
+  const uint32_t grid = persistent_grid((const void*)kernel, queue.capacity, tuning);
+  kernel<<<grid, kBlock, 0, stream>>>(S, queue, pass, records, stride, positive ? 1u : 0u, refill);
 }
 
 void launch_diagnostic(const SceneView& S, const FrameConst* fc, const uint32_t rect[4], uint32_t output,
