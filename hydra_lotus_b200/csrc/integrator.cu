@@ -1258,11 +1258,12 @@ uint32_t persistent_grid(const void* kernel, uint32_t capacity, const TraceTunin
   return std::max(1u, std::min(grid, (capacity + kBlock - 1) / kBlock));
 }
 
-uint32_t choose_wavefront_rounds(const uint32_t* counts, uint32_t resident, uint32_t max_bounces) {
+uint32_t choose_wavefront_rounds(const uint32_t* counts, uint32_t resident, uint32_t max_bounces, uint32_t samples,
+    uint32_t counted) {
   constexpr uint32_t kTailQueue = 65536;
-  const uint32_t below = std::max(resident, kTailQueue);
+  const uint64_t below = (uint64_t)std::max(resident, kTailQueue) * counted;
   for (uint32_t b = 1; b <= max_bounces; ++b)
-    if (counts[3 * b] < below) return b;
+    if ((uint64_t)counts[3 * b] * samples < below) return b;
   return max_bounces + 1;
 }
 

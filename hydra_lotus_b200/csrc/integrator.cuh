@@ -170,9 +170,11 @@ uint32_t wavefront_rounds(uint32_t max_bounces, bool count_visits, uint32_t requ
 // device at once (`resident`, at least 65,536), else every bounce. A round
 // over a queue that cannot fill the device once costs more than the tail
 // kernel's share of it (the reference's round scheduler stops at a
-// sixteenth of the camera rays instead). Results do not depend on it; only
-// the launch count does.
-uint32_t choose_wavefront_rounds(const uint32_t* counts, uint32_t resident, uint32_t max_bounces);
+// sixteenth of the camera rays instead). The counts are of `counted`
+// samples, the rounds for `samples`. Results do not depend on it; only the
+// launch count does.
+uint32_t choose_wavefront_rounds(const uint32_t* counts, uint32_t resident, uint32_t max_bounces,
+    uint32_t samples = 1, uint32_t counted = 1);
 
 // Threads of the extension kernel resident on the device at once.
 uint32_t extension_resident_threads();

@@ -42,6 +42,12 @@ struct DeviceArray {
     if (e != cudaSuccess || n == 0) return e;
     return cudaMemcpyAsync(ptr, host, n * sizeof(T), cudaMemcpyHostToDevice, s);
   }
+  // Room for at least n elements; `grown` tells that the array moved.
+  cudaError_t grow(size_t n, bool& grown) {
+    if (n <= count) return cudaSuccess;
+    grown = true;
+    return resize(n);
+  }
   void release() {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
@@ -631,14 +637,21 @@ LightTable build_light_table(const lotus_scene_desc& s, double env_mean) {
 
 }  // namespace
 
-// The longest chain of samples one RenderScene graph holds (two in flight
-// at a time): each sample has its own frame constants.
-constexpr uint32_t kMaxChain = 16;
+// The most waves one RenderScene graph chains (two in flight at a time):
+// each has its own frame constants.
+constexpr uint32_t kMaxChain = 4;
 // Samples one wavefront holds (a wave) unless lotus_cuda_options says
-// otherwise, and the most it may: the path state and queues have room for
-// the renderer's wave size times the target's pixels.
+// otherwise, and the most the options may ask for. Where eight samples of a
+// small target leave most of a launch to its ramp-up and drain and the tail
+// kernel most of the frame, a wave holds up to kMaxSmallWave samples of at
+// most kWavePaths paths together (2^21 paths: 344 MB of path state and
+// queues). Box room at 256 squared, 64 samples: 5.36 ms in eights, 5.07 with
+// waves of 2^20 paths, 4.59 with 2^21, 4.60 with 2^22; the texture fixture
+// at 161 squared, 128 samples: 4.58, 3.67, 3.08 and 3.09 ms (its tail kernel
+// 2.53 -> 0.25).
 constexpr uint32_t kDefaultWave = 8;
-constexpr uint32_t kMaxWave = 8;
+constexpr uint32_t kMaxSmallWave = 64;
+constexpr uint64_t kWavePaths = 1ull << 21;
 
 // The resident scene as the incremental updates need it: each geometry's
 // arrays (owned copies; `geometries` points into them), its box and its
@@ -757,7 +770,7 @@ struct Renderer {
   // before and read after each frame.
   DeviceArray<uint32_t> walk_failure;
   uint32_t step_limit = kMaxTraversalSteps;
-  uint32_t wave = kDefaultWave;  // samples per wavefront (lotus_cuda_options::samples_per_wave)
+  uint32_t wave = 0;  // samples per wavefront (lotus_cuda_options::samples_per_wave; 0: chosen by the target)
   // Profiling events, created on first use.
   std::vector<cudaEvent_t> profile_events;
   std::vector<int> profile_kinds;
@@ -821,31 +834,39 @@ struct Renderer {
   uint32_t cache_pixels = 0;
   uint32_t cache_generation = 0;  // bumped by every configuration
 
-  // The wavefront sample as a CUDA graph, and chains of two samples in
-  // flight: one instantiated graph per chain length (2, 4, .. kMaxChain,
-  // at index length / 2), all of one key, so that a call whose remainder
-  // makes a short chain does not re-instantiate the long one.
-  cudaGraphExec_t graph = nullptr;
-  cudaGraphExec_t graph_chains[3 * (kMaxChain / 2 + 1)] = {};
+  // Captured CUDA graphs: a sample (wave and count 0), or a chain of `count`
+  // waves of `wave` samples. The least recently launched one is given up
+  // for a new one.
   struct GraphKey {
     uint64_t scene_generation;
     uint32_t width, height, max_bounces;
     uint32_t rect[4];
-    uint32_t cache;  // the radiance cache's configuration count (0: off)
-    uint32_t rounds; // wavefront rounds before the tail kernel
+    uint32_t cache;   // the radiance cache's configuration count (0: off)
+    uint32_t rounds;  // wavefront rounds before the tail kernel
+    uint32_t wave, count;
+    uint32_t buffers; // buffer_generation: the arrays the graph's launches name
     bool operator==(const GraphKey& o) const { return std::memcmp(this, &o, sizeof(GraphKey)) == 0; }
-  } graph_key{}, graph_chain_key{};
-  // Rounds before the tail, chosen (choose_wavefront_rounds) from the queue
-  // counts of the first sample rendered with `rounds_key` (its rounds field
-  // 0), for RenderScene and for the temporal frames.
+  };
+  struct CapturedGraph {
+    GraphKey key{};
+    cudaGraphExec_t exec = nullptr;
+    uint64_t used = 0;
+  };
+  std::array<CapturedGraph, 8> graphs;
+  uint64_t graph_clock = 0;
+  uint32_t buffer_generation = 0;  // bumped when a target, path state or queue array moves
+  // Rounds before the tail are chosen (choose_wavefront_rounds) from the
+  // queue counts of the first wave rendered with `rounds_key` (its rounds,
+  // wave, count and buffers 0), which held `rounds_samples` samples; for the
+  // temporal frames from their first sample's.
   GraphKey rounds_key{}, temporal_rounds_key{};
-  uint32_t auto_rounds = 0, temporal_auto_rounds = 0;
+  std::vector<uint32_t> rounds_counts;
+  uint32_t rounds_samples = 0, temporal_auto_rounds = 0;
 
   ~Renderer() {
     for (cudaEvent_t e : profile_events) cudaEventDestroy(e);
-    if (graph) cudaGraphExecDestroy(graph);
-    for (cudaGraphExec_t g : graph_chains)
-      if (g) cudaGraphExecDestroy(g);
+    for (const CapturedGraph& g : graphs)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
     for (cudaEvent_t e : {ev_fork, ev_join})
       if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ev_sample_done) cudaEventDestroy(e);
@@ -1760,65 +1781,67 @@ int32_t update_geometry(Renderer& R, uint32_t geometry, const float* positions, 
   return LOTUS_PASS;
 }
 
-bool ensure_targets(Renderer& R, uint32_t w, uint32_t h, bool wavefront, std::string& detail) {
+// The targets and, for the queue kernels, a path state and queues of at
+// least `slots` paths, which a larger target or wave grows and the others
+// keep.
+bool ensure_targets(Renderer& R, uint32_t w, uint32_t h, size_t slots, std::string& detail) {
   const size_t n = (size_t)w * h;
+  bool moved = false;
   if (R.width != w || R.height != h) {
     R.accum.release();
     R.color.release();
     R.depth.release();
     R.depth_valid = false;
     R.depth_fresh = true;
-    R.path_origin.release(); R.path_direction.release(); R.path_throughput.release();
-    R.path_radiance.release(); R.path_hit.release();
-    R.queue_ray0.release(); R.queue_ray1.release(); R.queue_hit.release();
-    R.sq_o.release(); R.sq_d.release(); R.sq_fl.release(); R.sq_thr.release();
-    R.sort_keys.release(); R.sort_queue.release(); R.sort_bins.release();
-    R.path_origin2.release(); R.path_direction2.release(); R.path_throughput2.release();
-    R.path_radiance2.release(); R.path_hit2.release();
-    R.queue_ray02.release(); R.queue_ray12.release(); R.queue_hit2.release();
-    R.sq_o2.release(); R.sq_d2.release(); R.sq_fl2.release(); R.sq_thr2.release();
-    R.sort_keys2.release(); R.sort_queue2.release(); R.sort_bins2.release();
     R.width = w;
     R.height = h;
     R.key_valid = false;
+    moved = true;
   }
-  if (!R.ok(R.accum.resize(n), "accumulation", detail) || !R.ok(R.color.resize(n), "colour", detail) ||
-      !R.ok(R.depth.resize(n), "depth", detail) ||
-      !R.ok(R.counts.resize(kQueueCounterWords * (LOTUS_MAX_BOUNCES + 2)), "queue counts", detail) ||
-      !R.ok(R.frame_const.resize(kMaxChain), "frame constants", detail) ||
-      !R.ok(R.totals.resize(1), "ray totals", detail))
-    return false;
-  if (wavefront) {
-    // Room for a wave of the renderer's wave size.
-    const size_t w = (size_t)R.wave * n;
-    if (!R.ok(R.path_origin.resize(w), "path state", detail) ||
-        !R.ok(R.path_direction.resize(w), "path state", detail) ||
-        !R.ok(R.path_throughput.resize(w), "path state", detail) ||
-        !R.ok(R.path_radiance.resize(w), "path state", detail) ||
-        !R.ok(R.path_hit.resize(w), "path state", detail) ||
-        !R.ok(R.queue_ray0.resize(w), "queues", detail) || !R.ok(R.queue_ray1.resize(w), "queues", detail) ||
-        !R.ok(R.queue_hit.resize(w), "queues", detail) || !R.ok(R.sq_o.resize(w), "shadow queue", detail) ||
-        !R.ok(R.sq_d.resize(w), "shadow queue", detail) || !R.ok(R.sq_fl.resize(w), "shadow queue", detail) ||
-        !R.ok(R.sq_thr.resize(w), "shadow queue", detail) || !R.ok(R.sort_keys.resize(w), "queue keys", detail) ||
-        !R.ok(R.sort_queue.resize(w), "queue keys", detail) ||
-        !R.ok(R.sort_bins.resize(kSortBinWords), "queue keys", detail))
-      return false;
-  }
-  return true;
+  bool ok = R.ok(R.accum.resize(n), "accumulation", detail) && R.ok(R.color.resize(n), "colour", detail) &&
+            R.ok(R.depth.resize(n), "depth", detail) &&
+            R.ok(R.counts.resize(kQueueCounterWords * (LOTUS_MAX_BOUNCES + 2)), "queue counts", detail) &&
+            R.ok(R.frame_const.resize(1 + kMaxChain), "frame constants", detail) &&
+            R.ok(R.totals.resize(1), "ray totals", detail);
+  if (ok && slots)
+    ok = R.ok(R.path_origin.grow(slots, moved), "path state", detail) &&
+         R.ok(R.path_direction.grow(slots, moved), "path state", detail) &&
+         R.ok(R.path_throughput.grow(slots, moved), "path state", detail) &&
+         R.ok(R.path_radiance.grow(slots, moved), "path state", detail) &&
+         R.ok(R.path_hit.grow(slots, moved), "path state", detail) &&
+         R.ok(R.queue_ray0.grow(slots, moved), "queues", detail) &&
+         R.ok(R.queue_ray1.grow(slots, moved), "queues", detail) &&
+         R.ok(R.queue_hit.grow(slots, moved), "queues", detail) &&
+         R.ok(R.sq_o.grow(slots, moved), "shadow queue", detail) &&
+         R.ok(R.sq_d.grow(slots, moved), "shadow queue", detail) &&
+         R.ok(R.sq_fl.grow(slots, moved), "shadow queue", detail) &&
+         R.ok(R.sq_thr.grow(slots, moved), "shadow queue", detail) &&
+         R.ok(R.sort_keys.grow(slots, moved), "queue keys", detail) &&
+         R.ok(R.sort_queue.grow(slots, moved), "queue keys", detail) &&
+         R.ok(R.sort_bins.resize(kSortBinWords), "queue keys", detail);
+  if (moved) ++R.buffer_generation;
+  return ok;
 }
 
-// The second path state and queue set (two samples in flight).
+// The second path state and queue set (two waves in flight).
 bool ensure_pair_buffers(Renderer& R, size_t n, std::string& detail) {
-  return R.ok(R.path_origin2.resize(n), "path state", detail) && R.ok(R.path_direction2.resize(n), "path state", detail) &&
-         R.ok(R.path_throughput2.resize(n), "path state", detail) &&
-         R.ok(R.path_radiance2.resize(n), "path state", detail) && R.ok(R.path_hit2.resize(n), "path state", detail) &&
-         R.ok(R.queue_ray02.resize(n), "queues", detail) && R.ok(R.queue_ray12.resize(n), "queues", detail) &&
-         R.ok(R.queue_hit2.resize(n), "queues", detail) && R.ok(R.sq_o2.resize(n), "shadow queue", detail) &&
-         R.ok(R.sq_d2.resize(n), "shadow queue", detail) && R.ok(R.sq_fl2.resize(n), "shadow queue", detail) &&
-         R.ok(R.sq_thr2.resize(n), "shadow queue", detail) &&
-         R.ok(R.sort_keys2.resize(n), "queue keys", detail) && R.ok(R.sort_queue2.resize(n), "queue keys", detail) &&
-         R.ok(R.sort_bins2.resize(kSortBinWords), "queue keys", detail) &&
-         R.ok(R.counts2.resize(kQueueCounterWords * (LOTUS_MAX_BOUNCES + 2)), "queue counts", detail);
+  bool moved = false;
+  const bool ok =
+      R.ok(R.path_origin2.grow(n, moved), "path state", detail) &&
+      R.ok(R.path_direction2.grow(n, moved), "path state", detail) &&
+      R.ok(R.path_throughput2.grow(n, moved), "path state", detail) &&
+      R.ok(R.path_radiance2.grow(n, moved), "path state", detail) &&
+      R.ok(R.path_hit2.grow(n, moved), "path state", detail) &&
+      R.ok(R.queue_ray02.grow(n, moved), "queues", detail) && R.ok(R.queue_ray12.grow(n, moved), "queues", detail) &&
+      R.ok(R.queue_hit2.grow(n, moved), "queues", detail) && R.ok(R.sq_o2.grow(n, moved), "shadow queue", detail) &&
+      R.ok(R.sq_d2.grow(n, moved), "shadow queue", detail) && R.ok(R.sq_fl2.grow(n, moved), "shadow queue", detail) &&
+      R.ok(R.sq_thr2.grow(n, moved), "shadow queue", detail) &&
+      R.ok(R.sort_keys2.grow(n, moved), "queue keys", detail) &&
+      R.ok(R.sort_queue2.grow(n, moved), "queue keys", detail) &&
+      R.ok(R.sort_bins2.resize(kSortBinWords), "queue keys", detail) &&
+      R.ok(R.counts2.resize(kQueueCounterWords * (LOTUS_MAX_BOUNCES + 2)), "queue counts", detail);
+  if (moved) ++R.buffer_generation;
+  return ok;
 }
 
 // The radiance cache's queues for targets of `pixels` pixels: a query per
@@ -1902,6 +1925,18 @@ namespace {
 
 using namespace lotus;
 
+// The samples a call that adds `samples` runs in one wave: the options', or
+// kDefaultWave, doubled while kWavePaths and kMaxSmallWave allow it and two
+// such waves still fit into the call (two are in flight at a time); halved
+// while the call adds fewer.
+uint32_t call_wave(const Renderer& R, uint32_t pixels, uint32_t samples) {
+  uint32_t wave = R.wave ? R.wave : kDefaultWave;
+  if (R.wave == 0)
+    while (wave < kMaxSmallWave && 2ull * wave * pixels <= kWavePaths && 4ull * wave <= samples) wave *= 2;
+  while (wave > 1 && wave > samples) wave /= 2;
+  return wave;
+}
+
 int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, float* color_out) {
   std::string detail;
   auto fail = [&](const std::string& msg) {
@@ -1949,12 +1984,12 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   // and the sorted queues keep software traversal coherent. Below that the
   // frame is latency-bound and the per-thread loop (k_reference_pt) is
   // faster. The frame's evidence stays the reference integrator's.
-  const uint64_t launch_paths = (uint64_t)t.width * t.height *
-      std::min(std::max(d.frame_count, 1u), std::max(R.wave, 1u));
+  const uint32_t pixels = t.width * t.height;
+  const uint64_t launch_paths = (uint64_t)pixels * call_wave(R, pixels, d.frame_count);
   const bool queued = wavefront ||
       (st.integrator == LOTUS_INTEGRATOR_REFERENCE && st.light_sampling <= LOTUS_LIGHT_SAMPLING_MIS &&
        st.output == LOTUS_OUTPUT_RADIANCE && launch_paths >= extension_resident_threads());
-  if (!ensure_targets(R, t.width, t.height, queued, detail)) return poison(detail);
+  if (!ensure_targets(R, t.width, t.height, queued ? pixels : 0, detail)) return poison(detail);
   // The radiance cache serves the wavefront integrator's samples.
   const bool use_cache = wavefront && R.cache_enabled && R.cache.ready();
   if (use_cache && !ensure_cache_queues(R, t.width * t.height, detail)) return poison(detail);
@@ -2072,17 +2107,6 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
         (d.flags & LOTUS_FRAME_DEPTH_KEEP) == 0 || R.depth_fresh, t.clear_depth, s);
   R.depth_valid = want_depth;
   if (want_depth) R.depth_fresh = false;
-  PathState P{R.path_origin.ptr, R.path_direction.ptr, R.path_throughput.ptr, R.path_radiance.ptr, R.path_hit.ptr};
-  Queues Q;
-  Q.ray[0] = R.queue_ray0.ptr;
-  Q.ray[1] = R.queue_ray1.ptr;
-  Q.hit = R.queue_hit.ptr;
-  Q.shadow = ShadowQueue{R.sq_o.ptr, R.sq_d.ptr, R.sq_fl.ptr, R.sq_thr.ptr};
-  Q.counts = R.counts.ptr;
-  Q.capacity = t.width * t.height;
-  Q.keys = R.sort_keys.ptr;
-  Q.sorted = R.sort_queue.ptr;
-  Q.bins = R.sort_bins.ptr;
   const bool want_timings = (d.flags & LOTUS_FRAME_TIMINGS) != 0;
   const bool want_visits = (d.flags & LOTUS_FRAME_COUNT_VISITS) != 0;
   SampleProfile profile;
@@ -2108,7 +2132,7 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
       profile.visits = R.visits.ptr;
     }
   }
-  // The graph's key without its rounds, and the rounds this call runs.
+  // The graphs' key, without what a launch adds to it.
   Renderer::GraphKey gk{};
   gk.scene_generation = R.scene_generation;
   gk.width = t.width;
@@ -2116,24 +2140,31 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   gk.max_bounces = st.max_bounces;
   std::memcpy(gk.rect, rect, sizeof(rect));
   gk.cache = use_cache ? R.cache_generation : 0u;
-  TraceTuning tuning = R.tuning;
-  if (tuning.rounds == 0 && R.auto_rounds != 0 && R.rounds_key == gk) tuning.rounds = R.auto_rounds;
+  const Renderer::GraphKey shape_key = gk;
+  // The tuning of a wave of `samples` samples: its rounds as chosen from the
+  // first wave's queue counts, scaled to its size.
+  const bool rounds_known = R.tuning.rounds == 0 && R.rounds_samples != 0 && R.rounds_key == shape_key;
+  const bool choose_rounds = queued && R.tuning.rounds == 0 && !rounds_known;
+  auto wave_tuning = [&](uint32_t samples) {
+    TraceTuning tuning = R.tuning;
+    if (rounds_known)
+      tuning.rounds = choose_wavefront_rounds(R.rounds_counts.data(), extension_resident_threads(), st.max_bounces,
+          samples, R.rounds_samples);
+    return tuning;
+  };
   // The rounds the call's last sample ran (the frame result reports them).
-  uint32_t last_rounds = wavefront_rounds(st.max_bounces, want_visits, tuning.rounds, use_cache ? cq.bounce : 0u);
-  const bool choose_rounds = queued && R.tuning.rounds == 0 && !(R.rounds_key == gk);
+  uint32_t last_rounds =
+      wavefront_rounds(st.max_bounces, want_visits, wave_tuning(1).rounds, use_cache ? cq.bounce : 0u);
   // Samples in waves: where two or more are added without the radiance
   // cache (which trains between samples), the wavefront runs `wave` samples
-  // (the renderer's wave size, halved while the call adds fewer) as one
-  // wave, their paths in slots k * pixels + pixel of a path state R.wave
-  // times the target's size, so that every launch holds the wave's paths
-  // and pays its ramp-up and drain once for them. Chains of up to kMaxChain samples run two
-  // waves in flight: wave j on path state j % 2 and stream j % 2, each
-  // resolving (its samples in order) after wave j - 1, so that only the
-  // chain's last tail runs alone. A call's profiled part (timings or visit
-  // counts) is its last wave (or sample), run alone.
-  const uint32_t pixels = t.width * t.height;
-  uint32_t wave = std::max(R.wave, 1u);
-  while (wave > 1 && wave > to_add) wave /= 2;
+  // (call_wave; what is left over in smaller waves) as one wave, their paths
+  // in slots k * pixels + pixel of the path state, so that every launch holds
+  // the wave's paths and pays its ramp-up and drain once for them. Chains of
+  // up to kMaxChain waves run two in flight: wave j on path state j % 2 and
+  // stream j % 2, each resolving (its samples in order) after wave j - 1, so
+  // that only the chain's last tail runs alone. A call's profiled part
+  // (timings or visit counts) is its last wave (or sample), run alone.
+  const uint32_t wave = call_wave(R, pixels, to_add);
   const bool waves = queued && !use_cache && to_add >= 2 && wave >= 2;
   const uint32_t profiled_samples = (want_timings || want_visits) ? (waves ? wave : 1u) : 0u;
   const uint32_t chainable = waves ? submissions - profiled_samples : 0u;
@@ -2142,7 +2173,20 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
     if (!R.ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event", detail)) return poison(detail);
     R.ev_sample_done.push_back(e);
   }
-  if (chainable >= 2 * wave && !ensure_pair_buffers(R, (size_t)R.wave * pixels, detail)) return poison(detail);
+  if (waves && !ensure_targets(R, t.width, t.height, (size_t)wave * pixels, detail)) return poison(detail);
+  if (chainable >= 2 * wave && !ensure_pair_buffers(R, (size_t)wave * pixels, detail)) return poison(detail);
+  gk.buffers = R.buffer_generation;
+  PathState P{R.path_origin.ptr, R.path_direction.ptr, R.path_throughput.ptr, R.path_radiance.ptr, R.path_hit.ptr};
+  Queues Q;
+  Q.ray[0] = R.queue_ray0.ptr;
+  Q.ray[1] = R.queue_ray1.ptr;
+  Q.hit = R.queue_hit.ptr;
+  Q.shadow = ShadowQueue{R.sq_o.ptr, R.sq_d.ptr, R.sq_fl.ptr, R.sq_thr.ptr};
+  Q.counts = R.counts.ptr;
+  Q.capacity = pixels;
+  Q.keys = R.sort_keys.ptr;
+  Q.sorted = R.sort_queue.ptr;
+  Q.bins = R.sort_bins.ptr;
   PathState P2{R.path_origin2.ptr, R.path_direction2.ptr, R.path_throughput2.ptr, R.path_radiance2.ptr,
       R.path_hit2.ptr};
   Queues Q2 = Q;
@@ -2154,66 +2198,87 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   Q2.keys = R.sort_keys2.ptr;
   Q2.sorted = R.sort_queue2.ptr;
   Q2.bins = R.sort_bins2.ptr;
-  // A wave's queues hold both samples' paths.
-  Queues QW = Q, QW2 = Q2;
-  QW.capacity = QW2.capacity = wave * pixels;
   const uint32_t* last_counts = R.counts.ptr;  // the call's last launch's queue counts
   uint32_t last_wave = 1;                      // and the samples it held
   FrameConst* fc0 = R.frame_const.ptr;
+  // The instantiated graph of `key`, or the slot to put it into.
+  auto find_graph = [&](const Renderer::GraphKey& key) -> Renderer::CapturedGraph& {
+    Renderer::CapturedGraph* slot = &R.graphs[0];
+    for (Renderer::CapturedGraph& g : R.graphs) {
+      if (g.exec && g.key == key) {
+        slot = &g;
+        break;
+      }
+      if (g.used < slot->used) slot = &g;
+    }
+    if (slot->exec && !(slot->key == key)) {
+      cudaGraphExecDestroy(slot->exec);
+      slot->exec = nullptr;
+    }
+    slot->key = key;
+    slot->used = ++R.graph_clock;
+    return *slot;
+  };
+  auto end_capture = [&](Renderer::CapturedGraph& slot) {
+    cudaGraph_t g;
+    if (!R.ok(cudaStreamEndCapture(s, &g), "graph capture", detail)) return false;
+    const cudaError_t e = cudaGraphInstantiate(&slot.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) slot.exec = nullptr;
+    return R.ok(e, "graph instantiate", detail);
+  };
   cudaEventRecord(R.ev_start, s);
   for (uint32_t k = 0; k < submissions;) {
-    if (k + wave <= chainable) {
-      // A chain of `length` samples (a multiple of the wave, at most
-      // kMaxChain) in length / wave waves; wave j's frame constants are
+    uint32_t w = k < chainable ? wave : 1u;
+    while (w > 1 && w > chainable - k) w /= 2;
+    if (w > 1) {
+      // A chain of `count` waves of w samples; wave j's frame constants are
       // fc0's advanced by j waves.
-      const uint32_t length = std::min(kMaxChain, (chainable - k) / wave * wave);
-      const uint32_t count = length / wave;
+      const uint32_t count = w == wave ? std::min(kMaxChain, (chainable - k) / w) : 1u;
+      const TraceTuning tuning = wave_tuning(w);
       gk.rounds = wavefront_rounds(st.max_bounces, false, tuning.rounds, 0u);
-      if (!(R.graph_chain_key == gk)) {
-        for (cudaGraphExec_t& old : R.graph_chains)
-          if (old) {
-            cudaGraphExecDestroy(old);
-            old = nullptr;
-          }
-        R.graph_chain_key = gk;
-      }
-      // One graph per chain length and wave size (2, 4, 8).
-      const uint32_t shape = wave >= 8 ? 2u : wave >= 4 ? 1u : 0u;
-      cudaGraphExec_t& chain = R.graph_chains[shape * (kMaxChain / 2 + 1) + count];
-      if (!chain) {
-        cudaGraph_t g;
+      gk.wave = w;
+      gk.count = count;
+      Renderer::CapturedGraph& chain = find_graph(gk);
+      if (!chain.exec) {
+        Queues QW = Q, QW2 = Q2;
+        QW.capacity = QW2.capacity = w * pixels;
         if (!R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
           return poison(detail);
-        for (uint32_t j = 0; j < count; ++j) launch_wave_frame(fc0, fc0 + 1 + j, wave * j, wave, pixels, s);
-        cudaEventRecord(R.ev_fork, s);
-        cudaStreamWaitEvent(R.stream2, R.ev_fork, 0);
+        for (uint32_t j = 0; j < count; ++j) launch_wave_frame(fc0, fc0 + 1 + j, w * j, w, pixels, s);
+        if (count > 1) {
+          cudaEventRecord(R.ev_fork, s);
+          cudaStreamWaitEvent(R.stream2, R.ev_fork, 0);
+        }
         for (uint32_t j = 0; j < count; ++j) {
           const bool second = (j & 1u) != 0;
           launch_wavefront_sample(R.view, fc0 + 1 + j, rect, t.width, t.height, st.max_bounces, second ? P2 : P,
               second ? QW2 : QW, R.accum.ptr, R.color.ptr, R.totals.ptr, second ? R.stream2 : s, nullptr, tuning,
-              nullptr, j ? R.ev_sample_done[j - 1] : nullptr, wave);
+              nullptr, j ? R.ev_sample_done[j - 1] : nullptr, w);
           cudaEventRecord(R.ev_sample_done[j], second ? R.stream2 : s);
         }
-        cudaEventRecord(R.ev_join, R.stream2);
-        cudaStreamWaitEvent(s, R.ev_join, 0);
-        launch_advance_by(fc0, length, s);
-        if (!R.ok(cudaStreamEndCapture(s, &g), "graph capture", detail)) return poison(detail);
-        cudaError_t e = cudaGraphInstantiate(&chain, g, 0);
-        cudaGraphDestroy(g);
-        if (!R.ok(e, "graph instantiate", detail)) return poison(detail);
+        if (count > 1) {
+          cudaEventRecord(R.ev_join, R.stream2);
+          cudaStreamWaitEvent(s, R.ev_join, 0);
+        }
+        launch_advance_by(fc0, w * count, s);
+        if (!end_capture(chain)) return poison(detail);
       }
-      if (!R.ok(cudaGraphLaunch(chain, s), "graph launch", detail)) return poison(detail);
-      k += length;
+      if (!R.ok(cudaGraphLaunch(chain.exec, s), "graph launch", detail)) return poison(detail);
+      k += w * count;
       last_counts = ((count - 1) & 1u) ? R.counts2.ptr : R.counts.ptr;
-      last_wave = wave;
+      last_wave = w;
       last_rounds = gk.rounds;
       continue;
     }
     const bool profiled = profiled_samples != 0 && k + profiled_samples == submissions;
+    const TraceTuning tuning = wave_tuning(profiled ? profiled_samples : 1u);
     last_rounds = wavefront_rounds(st.max_bounces, profiled && want_visits, tuning.rounds, use_cache ? cq.bounce : 0u);
     last_counts = R.counts.ptr;
     if (profiled && profiled_samples > 1) {
       // The profiled last wave, run alone.
+      Queues QW = Q;
+      QW.capacity = wave * pixels;
       launch_wave_frame(fc0, fc0 + 1, 0, wave, pixels, s);
       launch_wavefront_sample(R.view, fc0 + 1, rect, t.width, t.height, st.max_bounces, P, QW, R.accum.ptr,
           R.color.ptr, R.totals.ptr, s, &profile, tuning, &cq, nullptr, wave);
@@ -2233,25 +2298,18 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
             &profile);
       launch_advance(R.frame_const.ptr, s);
     } else if (queued) {
-      gk.rounds = wavefront_rounds(st.max_bounces, false, tuning.rounds, use_cache ? cq.bounce : 0u);
-      if (!R.graph || !(R.graph_key == gk)) {
-        if (R.graph) {
-          cudaGraphExecDestroy(R.graph);
-          R.graph = nullptr;
-        }
-        cudaGraph_t g;
+      gk.rounds = last_rounds;
+      gk.wave = gk.count = 0;
+      Renderer::CapturedGraph& one = find_graph(gk);
+      if (!one.exec) {
         if (!R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
           return poison(detail);
         launch_wavefront_sample(R.view, R.frame_const.ptr, rect, t.width, t.height, st.max_bounces, P, Q,
             R.accum.ptr, R.color.ptr, R.totals.ptr, s, nullptr, tuning, &cq);
         launch_advance(R.frame_const.ptr, s);
-        if (!R.ok(cudaStreamEndCapture(s, &g), "graph capture", detail)) return poison(detail);
-        cudaError_t e = cudaGraphInstantiate(&R.graph, g, 0);
-        cudaGraphDestroy(g);
-        if (!R.ok(e, "graph instantiate", detail)) return poison(detail);
-        R.graph_key = gk;
+        if (!end_capture(one)) return poison(detail);
       }
-      if (!R.ok(cudaGraphLaunch(R.graph, s), "graph launch", detail)) return poison(detail);
+      if (!R.ok(cudaGraphLaunch(one.exec, s), "graph launch", detail)) return poison(detail);
     } else {
       launch_reference_pt(R.view, R.frame_const.ptr, rect, R.accum.ptr, R.color.ptr, R.totals.ptr, s);
       launch_advance(R.frame_const.ptr, s);
@@ -2343,9 +2401,9 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   }
   if (queued && to_add > 0) {
     if (choose_rounds) {
-      gk.rounds = 0;
-      R.rounds_key = gk;
-      R.auto_rounds = choose_wavefront_rounds(counts.data(), extension_resident_threads(), st.max_bounces);
+      R.rounds_key = shape_key;
+      R.rounds_counts = counts;
+      R.rounds_samples = last_wave;
     }
   }
   return LOTUS_PASS;
@@ -2415,7 +2473,7 @@ int32_t lotus_cuda_create(const lotus_cuda_options* options, lotus_cuda_renderer
                      options->wavefront_rounds > LOTUS_MAX_BOUNCES + 1 ||
                      (options->samples_per_wave != 0 && options->samples_per_wave != 1 &&
                       options->samples_per_wave != 2 && options->samples_per_wave != 4 &&
-                      options->samples_per_wave != kMaxWave))) {
+                      options->samples_per_wave != kDefaultWave))) {
     copy_detail(error, error_size,
         "trace_refill_below must be in 0..32, trace_blocks_per_sm in 0..64, wavefront_rounds in 0..1025 "
         "and samples_per_wave 0, 1, 2, 4 or 8");
@@ -2427,7 +2485,7 @@ int32_t lotus_cuda_create(const lotus_cuda_options* options, lotus_cuda_renderer
     R.tuning.blocks_per_sm = options->trace_blocks_per_sm;
     R.tuning.rounds = options->wavefront_rounds;
     if (options->traversal_step_limit) R.step_limit = options->traversal_step_limit;
-    if (options->samples_per_wave) R.wave = options->samples_per_wave;
+    R.wave = options->samples_per_wave;
   }
   std::string detail;
   if (!R.ok(cudaSetDevice(device), "cudaSetDevice", detail) ||
@@ -2837,7 +2895,7 @@ int32_t render_temporal(Renderer& R, const lotus_temporal_desc& td, lotus_frame_
   }
   Renderer::Temporal& T = R.temporal;
   const bool wavefront = st.integrator == LOTUS_INTEGRATOR_WAVEFRONT;
-  if (!ensure_targets(R, t.width, t.height, wavefront, detail)) return poison(detail);
+  if (!ensure_targets(R, t.width, t.height, wavefront ? (size_t)t.width * t.height : 0, detail)) return poison(detail);
   // Buffers.
   const size_t n = (size_t)t.width * t.height;
   if (T.width != t.width || T.height != t.height) {

@@ -416,10 +416,10 @@ typedef struct lotus_frame_result {
    * queued after the wavefront_rounds rounds, each followed to its end). */
   double tail_gpu_ms;
   /* The samples the call's last wavefront held: a call that adds two or
-   * more samples (without the radiance cache) runs them in waves of eight
-   * (lotus_cuda_options::samples_per_wave; halved while the call adds fewer)
-   * to a wavefront, and then the queue counts, the timings and the visit
-   * counts above are those of its last wave, its samples together. */
+   * more samples (without the radiance cache) runs them in waves
+   * (lotus_cuda_options::samples_per_wave; smaller ones for what is left
+   * over), and then the queue counts, the timings and the visit counts above
+   * are those of its last wave, its samples together. */
   uint32_t last_wave_samples;
   uint32_t reserved;
   /* With LOTUS_FRAME_TIMINGS: the device time spent putting the extension
@@ -461,9 +461,10 @@ typedef struct lotus_cuda_options {
   uint32_t traversal_step_limit;
   /* Samples a RenderScene call that adds several runs in one wavefront
    * (their paths side by side in one set of queues, so that each launch
-   * pays its ramp-up and drain once for all of them): 1, 2, 4 or 8; 0: 8.
-   * The path state and queues take this many times the target's pixels.
-   * Results do not depend on it. */
+   * pays its ramp-up and drain once for all of them): 1, 2, 4 or 8; 0: 8,
+   * and on small targets as many as keep 2^21 paths in a wave, up to 64. The
+   * path state and queues take this many times the target's pixels. Results
+   * do not depend on it. */
   uint32_t samples_per_wave;
 } lotus_cuda_options;
 
