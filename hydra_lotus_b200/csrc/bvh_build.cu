@@ -1,15 +1,15 @@
 // SPDX-License-Identifier: Apache-2.0
 // On-device BVH construction, replacing the driver's BLAS/TLAS builds. Two
-// builders: a binned-SAH builder that runs one BVH per CTA (all of a
-// scene's BLASes in one launch, and the TLAS), and, for meshes too large
-// for one CTA, a linear BVH (Karras, "Maximizing Parallelism in the
+// builders: a SAH builder of many BVHs at once (all of a scene's BLASes in
+// three launches, and the TLAS), and, for larger meshes, a linear BVH (Karras, "Maximizing Parallelism in the
 // Construction of BVHs, Octrees, and k-d Trees", HPG 2012) over 63-bit
 // Morton codes of the primitives' centroids, sorted by CUB's radix sort,
 // with bounds fitted bottom-up. The reference's builds are (backend/vulkan/gpu_scene.cpp:1899-1950, 2240-2322 in
 // hydra-lotus).
 #include "bvh_build.cuh"
 
-#include <cub/block/block_scan.cuh>
+#include <algorithm>
+
 #include <cub/device/device_radix_sort.cuh>
 
 namespace lotus {
@@ -70,9 +70,11 @@ __global__ void k_triangle_boxes(const float* __restrict__ positions,
 // world_from_object, widened by a relative margin.
 __global__ void k_instance_boxes(const InstanceShading* __restrict__ shade,
     const InstanceTraversal* __restrict__ trav, const BvhNode* __restrict__ blas, uint32_t n,
-    float4* __restrict__ lo, float4* __restrict__ hi, uint32_t* __restrict__ centroid_bounds) {
+    float4* __restrict__ lo, float4* __restrict__ hi, uint32_t* __restrict__ centroid_bounds,
+    uint32_t* __restrict__ idx) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (idx != nullptr) idx[i] = i;
   float l[3] = {kFloatMax, kFloatMax, kFloatMax}, h[3] = {-kFloatMax, -kFloatMax, -kFloatMax};
   const uint32_t root = trav[i].blas_root;
   if (root != (uint32_t)kEmptyChild) {
@@ -274,300 +276,598 @@ __global__ void k_write_triangles(const uint32_t* __restrict__ values,
 
 
 // ---------------------------------------------------------------------------
-// Binned-SAH builder: one CTA builds one BVH top-down (Wald, "On fast
-// Construction of SAH-based Bounding Volume Hierarchies", 2007), binning
-// centroids into 16 bins per axis in shared memory and partitioning the
-// primitive indices with a block-wide scan. Every BVH of a batch builds in
-// its own CTA, so a scene's BLASes build concurrently across the SMs.
+// SAH builder of a batch of BVHs (a scene's BLASes, or its TLAS), top-down
+// (Wald, "On fast Construction of SAH-based Bounding Volume Hierarchies",
+// 2007), each node built by as many threads as its primitives can use:
+//   - k_sah_large, one CTA per BVH: nodes of more than kSahMedium primitives;
+//   - k_sah_medium, one warp per subtree handed on by it: nodes of more than
+//     a warp's primitives. Both bin centroids into 16 bins per axis;
+//   - k_sah_small, one warp per subtree of at most 32 primitives: one
+//     primitive a lane and all of a level's nodes at once, with every split
+//     of the sorted centroids tried instead of bins.
+// The subtrees of all BVHs lie in one list per kernel, so that the GPU is
+// filled whatever the meshes' sizes. One CTA a BVH for all of its nodes (some
+// ten barriers each, five of six nodes over fewer than ten primitives) took
+// 45 ms for the sphere field's 320 meshes (1.07M triangles) and its 4,161
+// instances; the three take 0.32, 0.43 and 0.34 ms.
+//
+// A subtree over n primitives takes the n - 1 node slots from its own on:
+// its root, then the left child's, then the right child's, so that no
+// counter is needed and a subtree is contiguous.
 
-constexpr int kSahBlock = 256;
+constexpr int kSahBlock = 512;
 constexpr int kSahBins = 16;
 constexpr int kSahStack = 128;
+constexpr uint32_t kSahMedium = 512;
+constexpr uint32_t kSahSmall = 32;
+constexpr unsigned kAllLanes = 0xFFFFFFFFu;
 
-struct SahJob {
-  uint32_t prim_offset;  // first primitive in the batch's arrays
-  uint32_t count;
-  uint32_t node_base;    // first node slot
-  uint32_t leaf_base;    // first triangle-pool slot (BLAS)
-  uint32_t leaf_size;    // most primitives per leaf
-  uint32_t leaves_are_values;  // TLAS: leaves hold the primitive index itself
+// A node to build: its primitives [begin, end) of the job's and its slot.
+struct SahNode {
+  uint32_t job, begin, end, slot;
 };
 
+// The lists between the kernels and their counters: nodes appended, nodes
+// taken, and errors.
+struct SahLists {
+  SahNode* medium;
+  SahNode* small;
+  uint32_t* counters;
+};
+constexpr int kMediumCount = 0, kMediumTaken = 1, kSmallCount = 2, kSmallTaken = 3, kSahErrors = 4, kSahCounters = 5;
+
+// The threads that build one node together: a block or a warp.
+template <int kThreads>
+struct SahGroup {
+  static constexpr bool kWarp = kThreads == 32;
+  static __device__ __forceinline__ uint32_t rank() { return kWarp ? threadIdx.x & 31u : threadIdx.x; }
+  static __device__ __forceinline__ void sync() {
+    if (kWarp) __syncwarp();
+    else __syncthreads();
+  }
+};
+
+template <int kThreads>
 struct SahShared {
-  uint32_t bin_count[3][kSahBins];
-  uint32_t bin_lo[3][kSahBins][3];
-  uint32_t bin_hi[3][kSahBins][3];
-  uint32_t cb[6];        // centroid bounds (ordered)
-  uint32_t nb[6];        // node bounds (ordered)
-  uint32_t stack_begin[kSahStack], stack_end[kSahStack], stack_node[kSahStack];
-  int sp;
-  uint32_t next_node;
-  uint32_t begin, end, node;
-  int best_axis, best_split;
+  uint32_t count[3][kSahBins];
+  uint32_t lo[3][3][kSahBins];  // [binned axis][component][bin], ordered floats
+  uint32_t hi[3][3][kSahBins];
+  uint32_t bounds[12];          // centroid bounds; the halves' where no axis separates them
   float best_cost[3];
   int split_at[3];
-  uint32_t left_total;
-  uint32_t error;
-  uint32_t done;
+  uint32_t left_count[3];
+  float box[3][12];             // the children's boxes of each axis's best split
+  uint32_t warp_left[kThreads / 32];
+  uint32_t begin, end, slot;
 };
 
-__global__ void __launch_bounds__(kSahBlock) k_sah_build(const SahJob* __restrict__ jobs,
-    const float4* __restrict__ plo, const float4* __restrict__ phi, uint32_t* __restrict__ idx,
-    uint32_t* __restrict__ scratch, BvhNode* __restrict__ nodes, uint32_t* __restrict__ errors) {
-  using BlockScan = cub::BlockScan<uint32_t, kSahBlock>;
-  __shared__ typename BlockScan::TempStorage scan_storage;
-  __shared__ SahShared sh;
-  const SahJob job = jobs[blockIdx.x];
-  const uint32_t tid = threadIdx.x;
-  uint32_t* index = idx + job.prim_offset;
-  uint32_t* tmp = scratch + job.prim_offset;
-  if (job.count == 0) return;
-  if (tid == 0) {
-    sh.sp = 0;
-    sh.next_node = 1;
-    sh.error = 0;
-    sh.stack_begin[0] = 0;
-    sh.stack_end[0] = job.count;
-    sh.stack_node[0] = 0;
-    sh.sp = 1;
+__device__ __forceinline__ float sah_half_area(const float* lo, const float* hi) {
+  const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
+  return dx * dy + dy * dz + dz * dx;
+}
+
+// The reference of a child over [begin, end): a leaf, or the node at `slot`.
+__device__ __forceinline__ int32_t sah_child(const SahJob& job, const uint32_t* index, uint32_t begin, uint32_t end,
+    uint32_t slot, int32_t& count) {
+  count = end - begin <= job.leaf_size ? (int32_t)(end - begin) : 0;
+  if (count == 0) return (int32_t)(job.node_base + slot);
+  return job.leaves_are_values ? ~(int32_t)index[begin] : ~(int32_t)(job.leaf_base + begin);
+}
+
+__device__ __forceinline__ void sah_write_node(BvhNode* nodes, const SahJob& job, const uint32_t* index,
+    uint32_t begin, uint32_t mid, uint32_t end, uint32_t slot, const float* box) {
+  int32_t n0, n1;
+  const int32_t c0 = sah_child(job, index, begin, mid, slot + 1, n0);
+  const int32_t c1 = sah_child(job, index, mid, end, slot + (mid - begin), n1);
+  BvhNode nd;
+  nd.x = make_float4(box[0], box[3], box[6], box[9]);
+  nd.y = make_float4(box[1], box[4], box[7], box[10]);
+  nd.z = make_float4(box[2], box[5], box[8], box[11]);
+  nd.c = make_int4(c0, c1, n0, n1);
+  nodes[job.node_base + slot] = nd;
+}
+
+// The best split of one axis's bins, by the 16 lanes of a half warp (every
+// lane of the warp takes part): prefix and suffix boxes by scans. Lane 0 of
+// the half writes it down.
+template <int kThreads>
+__device__ __forceinline__ void sah_sweep(SahShared<kThreads>& sh, int axis, bool separates) {
+  const unsigned bin = threadIdx.x & 15u;
+  float l[3], h[3], rl[3], rh[3];
+  uint32_t left = sh.count[axis][bin], right = left;
+  for (int c = 0; c < 3; ++c) {
+    l[c] = rl[c] = left ? unordered(sh.lo[axis][c][bin]) : INFINITY;
+    h[c] = rh[c] = left ? unordered(sh.hi[axis][c][bin]) : -INFINITY;
   }
-  __syncthreads();
+#pragma unroll
+  for (unsigned off = 1; off < 16; off <<= 1) {
+    const uint32_t ln = __shfl_up_sync(kAllLanes, left, off, 16), rn = __shfl_down_sync(kAllLanes, right, off, 16);
+    const bool up = bin >= off, down = bin + off < 16;
+    left += up ? ln : 0u;
+    right += down ? rn : 0u;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float a = __shfl_up_sync(kAllLanes, l[c], off, 16), b = __shfl_up_sync(kAllLanes, h[c], off, 16);
+      const float d = __shfl_down_sync(kAllLanes, rl[c], off, 16), e = __shfl_down_sync(kAllLanes, rh[c], off, 16);
+      if (up) { l[c] = fminf(l[c], a); h[c] = fmaxf(h[c], b); }
+      if (down) { rl[c] = fminf(rl[c], d); rh[c] = fmaxf(rh[c], e); }
+    }
+  }
+  // The right side of a split after this bin begins at the next one.
+  right = __shfl_down_sync(kAllLanes, right, 1, 16);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    rl[c] = __shfl_down_sync(kAllLanes, rl[c], 1, 16);
+    rh[c] = __shfl_down_sync(kAllLanes, rh[c], 1, 16);
+  }
+  float cost = INFINITY;
+  if (separates && bin < 15 && left != 0 && right != 0)
+    cost = sah_half_area(l, h) * (float)left + sah_half_area(rl, rh) * (float)right;
+  float best = cost;
+  unsigned at = bin;
+#pragma unroll
+  for (unsigned off = 8; off >= 1; off >>= 1) {
+    const float other = __shfl_xor_sync(kAllLanes, best, off, 16);
+    const unsigned other_at = __shfl_xor_sync(kAllLanes, at, off, 16);
+    if (other < best || (other == best && other_at < at)) { best = other; at = other_at; }
+  }
+  if (bin == at) {
+    sh.best_cost[axis] = best;
+    sh.split_at[axis] = best < INFINITY ? (int)bin : -1;
+    sh.left_count[axis] = left;
+    for (int c = 0; c < 3; ++c) {
+      sh.box[axis][c] = l[c];
+      sh.box[axis][3 + c] = h[c];
+      sh.box[axis][6 + c] = rl[c];
+      sh.box[axis][9 + c] = rh[c];
+    }
+  }
+}
+
+// Builds one node: splits [begin, end) of the job's primitives (index, with
+// tmp as scratch) at the cheapest plane between bins, the order within each
+// side kept, and writes the node. Returns the first primitive of the right
+// side. Group-uniform; ends with the group in step.
+template <int kThreads>
+__device__ __forceinline__ uint32_t sah_split(const SahJob& job, uint32_t begin, uint32_t end, uint32_t slot,
+    const float4* __restrict__ plo, const float4* __restrict__ phi, uint32_t* index, uint32_t* tmp, BvhNode* nodes,
+    SahShared<kThreads>& sh) {
+  using G = SahGroup<kThreads>;
+  const uint32_t rank = G::rank();
+  const unsigned lane = threadIdx.x & 31u;
+  if (rank < 12) sh.bounds[rank] = rank % 6 < 3 ? 0xFFFFFFFFu : 0u;
+  for (uint32_t k = rank; k < 3 * kSahBins; k += kThreads) {
+    const uint32_t a = k / kSahBins, b = k % kSahBins;
+    sh.count[a][b] = 0;
+    for (int c = 0; c < 3; ++c) {
+      sh.lo[a][c][b] = 0xFFFFFFFFu;
+      sh.hi[a][c][b] = 0u;
+    }
+  }
+  G::sync();
+  // Centroid bounds: per thread, per warp, then one atomic a warp and bound.
+  uint32_t cl[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, ch[3] = {0u, 0u, 0u};
+  for (uint32_t i = begin + rank; i < end; i += kThreads) {
+    const uint32_t p = job.prim_offset + index[i];
+    const float4 l = plo[p], h = phi[p];
+    const uint32_t c[3] = {ordered(0.5f * (l.x + h.x)), ordered(0.5f * (l.y + h.y)), ordered(0.5f * (l.z + h.z))};
+    for (int a = 0; a < 3; ++a) {
+      cl[a] = min(cl[a], c[a]);
+      ch[a] = max(ch[a], c[a]);
+    }
+  }
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t l = __reduce_min_sync(kAllLanes, cl[a]), h = __reduce_max_sync(kAllLanes, ch[a]);
+    if (lane == 0) {
+      atomicMin(&sh.bounds[a], l);
+      atomicMax(&sh.bounds[3 + a], h);
+    }
+  }
+  G::sync();
+  float cmin[3], scale[3];
+  for (int a = 0; a < 3; ++a) {
+    cmin[a] = unordered(sh.bounds[a]);
+    const float extent = unordered(sh.bounds[3 + a]) - cmin[a];
+    scale[a] = extent > 0.0f ? float(kSahBins) / extent : 0.0f;
+  }
+  auto bin_of = [&](float lo, float hi, int a) {
+    // Each operation rounded by itself: the partition has to find the very
+    // bins that were counted.
+    const float c = __fmul_rn(0.5f, __fadd_rn(lo, hi));
+    return min(kSahBins - 1, max(0, (int)__fmul_rn(__fsub_rn(c, cmin[a]), scale[a])));
+  };
+  for (uint32_t i = begin + rank; i < end; i += kThreads) {
+    const uint32_t p = job.prim_offset + index[i];
+    const float4 l = plo[p], h = phi[p];
+    const uint32_t ol[3] = {ordered(l.x), ordered(l.y), ordered(l.z)}, oh[3] = {ordered(h.x), ordered(h.y), ordered(h.z)};
+    const int b[3] = {bin_of(l.x, h.x, 0), bin_of(l.y, h.y, 1), bin_of(l.z, h.z, 2)};
+    for (int a = 0; a < 3; ++a) {
+      atomicAdd(&sh.count[a][b[a]], 1u);
+      for (int c = 0; c < 3; ++c) {
+        atomicMin(&sh.lo[a][c][b[a]], ol[c]);
+        atomicMax(&sh.hi[a][c][b[a]], oh[c]);
+      }
+    }
+  }
+  G::sync();
+  // Half warps sweep an axis each: a block's first two warps, or a warp twice.
+  if (G::kWarp) {
+    const int a = (int)(lane >> 4);
+    sah_sweep(sh, a, (a ? scale[1] : scale[0]) > 0.0f);
+    sah_sweep(sh, 2, scale[2] > 0.0f);
+  } else if (threadIdx.x < 64) {
+    const int a = min((int)(threadIdx.x >> 4), 2);
+    sah_sweep(sh, a, (a == 0 ? scale[0] : a == 1 ? scale[1] : scale[2]) > 0.0f);
+  }
+  G::sync();
+  int axis = -1;
+  float best = INFINITY;
+  for (int a = 0; a < 3; ++a)
+    if (sh.split_at[a] >= 0 && sh.best_cost[a] < best) {
+      best = sh.best_cost[a];
+      axis = a;
+    }
+  uint32_t mid;
+  if (axis < 0) {
+    // Coincident centroids: the list's halves, whose boxes no bins hold.
+    mid = begin + (end - begin) / 2;
+    for (int side = 0; side < 2; ++side) {
+      G::sync();
+      if (rank < 6) sh.bounds[rank] = rank < 3 ? 0xFFFFFFFFu : 0u;
+      G::sync();
+      for (uint32_t i = (side ? mid : begin) + rank; i < (side ? end : mid); i += kThreads) {
+        const float4 l = plo[job.prim_offset + index[i]], h = phi[job.prim_offset + index[i]];
+        atomicMin(&sh.bounds[0], ordered(l.x)); atomicMin(&sh.bounds[1], ordered(l.y)); atomicMin(&sh.bounds[2], ordered(l.z));
+        atomicMax(&sh.bounds[3], ordered(h.x)); atomicMax(&sh.bounds[4], ordered(h.y)); atomicMax(&sh.bounds[5], ordered(h.z));
+      }
+      G::sync();
+      if (rank < 6) sh.box[0][6 * side + rank] = unordered(sh.bounds[rank]);
+    }
+    axis = 0;
+  } else {
+    const int split = sh.split_at[axis];
+    const uint32_t left_total = sh.left_count[axis];
+    mid = begin + left_total;
+    uint32_t left_before = 0;  // lefts of the tiles done
+    for (uint32_t t0 = begin; t0 < end; t0 += kThreads) {
+      const uint32_t i = t0 + rank;
+      bool left = false;
+      uint32_t v = 0;
+      if (i < end) {
+        v = index[i];
+        const float4 l = plo[job.prim_offset + v], h = phi[job.prim_offset + v];
+        left = (axis == 0 ? bin_of(l.x, h.x, 0) : axis == 1 ? bin_of(l.y, h.y, 1) : bin_of(l.z, h.z, 2)) <= split;
+      }
+      const unsigned mask = __ballot_sync(kAllLanes, left);
+      uint32_t before = left_before + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+      if (G::kWarp) {
+        left_before += (uint32_t)__popc(mask);
+      } else {
+        G::sync();
+        if (lane == 0) sh.warp_left[threadIdx.x >> 5] = (uint32_t)__popc(mask);
+        G::sync();
+        for (uint32_t w = 0; w < kThreads / 32; ++w) {
+          const uint32_t n = sh.warp_left[w];
+          if (w < threadIdx.x >> 5) before += n;
+          left_before += n;
+        }
+      }
+      if (i < end) tmp[left ? begin + before : mid + (i - begin - before)] = v;
+    }
+    G::sync();
+    for (uint32_t i = begin + rank; i < end; i += kThreads) index[i] = tmp[i];
+  }
+  G::sync();
+  if (rank == 0) sah_write_node(nodes, job, index, begin, mid, end, slot, sh.box[axis]);
+  G::sync();
+  return mid;
+}
+
+// Where a child that is no leaf is built: true when the caller builds it.
+__device__ __forceinline__ bool sah_keep(const SahJob& job, uint32_t job_index, uint32_t begin, uint32_t end,
+    uint32_t slot, uint32_t above, const SahLists& lists, bool write) {
+  const uint32_t n = end - begin;
+  if (n <= job.leaf_size) return false;
+  if (n > above) return true;
+  if (write) {
+    const bool small = n <= kSahSmall;
+    (small ? lists.small : lists.medium)[atomicAdd(&lists.counters[small ? kSmallCount : kMediumCount], 1u)] =
+        SahNode{job_index, begin, end, slot};
+  }
+  return false;
+}
+
+__global__ void __launch_bounds__(kSahBlock) k_sah_large(const SahJob* __restrict__ jobs,
+    const float4* __restrict__ plo, const float4* __restrict__ phi, uint32_t* __restrict__ idx,
+    uint32_t* __restrict__ scratch, BvhNode* __restrict__ nodes, SahLists lists) {
+  __shared__ SahShared<kSahBlock> sh;
+  __shared__ uint32_t stack[kSahStack][3];
+  const SahJob job = jobs[blockIdx.x];
+  uint32_t* index = idx + job.prim_offset;
+  if (job.count == 0) return;
   // Small sets: one leaf under the root, its second child empty.
   if (job.count <= job.leaf_size) {
-    if (tid < 6) sh.nb[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
-    __syncthreads();
-    for (uint32_t i = tid; i < job.count; i += blockDim.x) {
-      const float4 l = plo[job.prim_offset + index[i]], h = phi[job.prim_offset + index[i]];
-      atomicMin(&sh.nb[0], ordered(l.x)); atomicMin(&sh.nb[1], ordered(l.y)); atomicMin(&sh.nb[2], ordered(l.z));
-      atomicMax(&sh.nb[3], ordered(h.x)); atomicMax(&sh.nb[4], ordered(h.y)); atomicMax(&sh.nb[5], ordered(h.z));
+    if (threadIdx.x != 0) return;
+    float l[3] = {kFloatMax, kFloatMax, kFloatMax}, h[3] = {-kFloatMax, -kFloatMax, -kFloatMax};
+    for (uint32_t i = 0; i < job.count; ++i) {
+      const float4 a = plo[job.prim_offset + index[i]], b = phi[job.prim_offset + index[i]];
+      l[0] = fminf(l[0], a.x); l[1] = fminf(l[1], a.y); l[2] = fminf(l[2], a.z);
+      h[0] = fmaxf(h[0], b.x); h[1] = fmaxf(h[1], b.y); h[2] = fmaxf(h[2], b.z);
     }
-    __syncthreads();
-    if (tid == 0) {
-      BvhNode nd;
-      nd.x = make_float4(unordered(sh.nb[0]), unordered(sh.nb[3]), 0.0f, 0.0f);
-      nd.y = make_float4(unordered(sh.nb[1]), unordered(sh.nb[4]), 0.0f, 0.0f);
-      nd.z = make_float4(unordered(sh.nb[2]), unordered(sh.nb[5]), 0.0f, 0.0f);
-      const int32_t leaf = job.leaves_are_values ? ~(int32_t)index[0] : ~(int32_t)job.leaf_base;
-      nd.c = make_int4(leaf, kEmptyChild, (int32_t)job.count, 0);
-      nodes[job.node_base] = nd;
-    }
+    BvhNode nd;
+    nd.x = make_float4(l[0], h[0], 0.0f, 0.0f);
+    nd.y = make_float4(l[1], h[1], 0.0f, 0.0f);
+    nd.z = make_float4(l[2], h[2], 0.0f, 0.0f);
+    const int32_t leaf = job.leaves_are_values ? ~(int32_t)index[0] : ~(int32_t)job.leaf_base;
+    nd.c = make_int4(leaf, kEmptyChild, (int32_t)job.count, 0);
+    nodes[job.node_base] = nd;
     return;
   }
-  for (int guard = 0; guard < (int)(2 * job.count + 8); ++guard) {
-    // Thread 0 pops the next range; the barrier publishes it (and orders
-    // the pop after every thread's use of the previous node's state).
-    if (tid == 0) {
-      sh.done = sh.sp == 0 ? 1u : 0u;
-      if (sh.sp > 0) {
-        --sh.sp;
-        sh.begin = sh.stack_begin[sh.sp];
-        sh.end = sh.stack_end[sh.sp];
-        sh.node = sh.stack_node[sh.sp];
+  uint32_t begin = 0, end = job.count, slot = 0;
+  if (!sah_keep(job, blockIdx.x, begin, end, slot, kSahMedium, lists, threadIdx.x == 0)) return;
+  int sp = 0;
+  // Every step splits one node, of at most count - 1. The smaller side is
+  // built first, so that the stack holds at most one range per halving.
+  for (uint32_t step = 0; step < job.count; ++step) {
+    const uint32_t mid = sah_split<kSahBlock>(job, begin, end, slot, plo, phi, index, scratch + job.prim_offset, nodes, sh);
+    uint32_t r[2][3] = {{begin, mid, slot + 1}, {mid, end, slot + (mid - begin)}};
+    const bool keep[2] = {sah_keep(job, blockIdx.x, r[0][0], r[0][1], r[0][2], kSahMedium, lists, threadIdx.x == 0),
+        sah_keep(job, blockIdx.x, r[1][0], r[1][1], r[1][2], kSahMedium, lists, threadIdx.x == 0)};
+    int next = keep[0] ? 0 : keep[1] ? 1 : -1;
+    if (keep[0] && keep[1]) {
+      next = mid - begin <= end - mid ? 0 : 1;
+      if (sp >= kSahStack) {
+        if (threadIdx.x == 0) atomicAdd(&lists.counters[kSahErrors], 1u);
+        return;
       }
+      if (threadIdx.x < 3) stack[sp][threadIdx.x] = r[1 - next][threadIdx.x];
+      ++sp;
     }
     __syncthreads();
-    if (sh.done) break;
-    if (tid < 6) sh.cb[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
-    for (uint32_t k = tid; k < 3 * kSahBins; k += blockDim.x) {
-      const uint32_t a = k / kSahBins, b = k % kSahBins;
-      sh.bin_count[a][b] = 0;
-      for (int c = 0; c < 3; ++c) {
-        sh.bin_lo[a][b][c] = 0xFFFFFFFFu;
-        sh.bin_hi[a][b][c] = 0u;
-      }
-    }
-    __syncthreads();
-    const uint32_t begin = sh.begin, end = sh.end;
-    // Centroid bounds.
-    for (uint32_t i = begin + tid; i < end; i += blockDim.x) {
-      const uint32_t p = job.prim_offset + index[i];
-      const float4 l = plo[p], h = phi[p];
-      const float cx = 0.5f * (l.x + h.x), cy = 0.5f * (l.y + h.y), cz = 0.5f * (l.z + h.z);
-      atomicMin(&sh.cb[0], ordered(cx)); atomicMin(&sh.cb[1], ordered(cy)); atomicMin(&sh.cb[2], ordered(cz));
-      atomicMax(&sh.cb[3], ordered(cx)); atomicMax(&sh.cb[4], ordered(cy)); atomicMax(&sh.cb[5], ordered(cz));
-    }
-    __syncthreads();
-    float cmin[3], scale[3];
-    for (int a = 0; a < 3; ++a) {
-      cmin[a] = unordered(sh.cb[a]);
-      const float extent = unordered(sh.cb[3 + a]) - cmin[a];
-      scale[a] = extent > 0.0f ? float(kSahBins) / extent : 0.0f;
-    }
-    // Binning on all three axes.
-    for (uint32_t i = begin + tid; i < end; i += blockDim.x) {
-      const uint32_t p = job.prim_offset + index[i];
-      const float4 l = plo[p], h = phi[p];
-      const float c[3] = {0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z)};
-      for (int a = 0; a < 3; ++a) {
-        const int b = min(kSahBins - 1, max(0, (int)((c[a] - cmin[a]) * scale[a])));
-        atomicAdd(&sh.bin_count[a][b], 1u);
-        atomicMin(&sh.bin_lo[a][b][0], ordered(l.x)); atomicMin(&sh.bin_lo[a][b][1], ordered(l.y));
-        atomicMin(&sh.bin_lo[a][b][2], ordered(l.z));
-        atomicMax(&sh.bin_hi[a][b][0], ordered(h.x)); atomicMax(&sh.bin_hi[a][b][1], ordered(h.y));
-        atomicMax(&sh.bin_hi[a][b][2], ordered(h.z));
-      }
-    }
-    __syncthreads();
-    // The SAH sweep, one axis per thread.
-    if (tid < 3) {
-      const int a = tid;
-      float best = INFINITY;
-      int split = -1;
-      if (scale[a] > 0.0f) {
-        float right_area[kSahBins];
-        uint32_t right_count[kSahBins];
-        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        uint32_t cnt = 0;
-        for (int b = kSahBins - 1; b > 0; --b) {
-          if (sh.bin_count[a][b]) {
-            for (int c = 0; c < 3; ++c) {
-              lo[c] = fminf(lo[c], unordered(sh.bin_lo[a][b][c]));
-              hi[c] = fmaxf(hi[c], unordered(sh.bin_hi[a][b][c]));
-            }
-          }
-          cnt += sh.bin_count[a][b];
-          const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-          right_area[b] = cnt ? 2.0f * (dx * dy + dy * dz + dz * dx) : 0.0f;
-          right_count[b] = cnt;
-        }
-        lo[0] = lo[1] = lo[2] = INFINITY;
-        hi[0] = hi[1] = hi[2] = -INFINITY;
-        cnt = 0;
-        for (int b = 0; b < kSahBins - 1; ++b) {
-          if (sh.bin_count[a][b]) {
-            for (int c = 0; c < 3; ++c) {
-              lo[c] = fminf(lo[c], unordered(sh.bin_lo[a][b][c]));
-              hi[c] = fmaxf(hi[c], unordered(sh.bin_hi[a][b][c]));
-            }
-          }
-          cnt += sh.bin_count[a][b];
-          if (cnt == 0 || right_count[b + 1] == 0) continue;
-          const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-          const float cost = 2.0f * (dx * dy + dy * dz + dz * dx) * cnt + right_area[b + 1] * right_count[b + 1];
-          if (cost < best) {
-            best = cost;
-            split = b;
-          }
-        }
-      }
-      sh.best_cost[a] = best;
-      sh.split_at[a] = split;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int axis = -1;
-      float best = INFINITY;
-      for (int a = 0; a < 3; ++a)
-        if (sh.split_at[a] >= 0 && sh.best_cost[a] < best) {
-          best = sh.best_cost[a];
-          axis = a;
-        }
-      sh.best_axis = axis;
-      sh.best_split = axis >= 0 ? sh.split_at[axis] : -1;
-    }
-    __syncthreads();
-    const int axis = sh.best_axis, split = sh.best_split;
-    const uint32_t count = end - begin;
-    uint32_t mid;
-    if (axis < 0) {
-      mid = begin + count / 2;  // coincident centroids: split the list
+    if (next >= 0) {
+      begin = r[next][0];
+      end = r[next][1];
+      slot = r[next][2];
     } else {
-      // Stable partition: lefts to the front of tmp's range, rights after.
-      uint32_t left_base = 0;
-      uint32_t left_total = 0;
-      for (uint32_t t0 = begin; t0 < end; t0 += blockDim.x) {
-        const uint32_t i = t0 + tid;
-        uint32_t goes_left = 0;
-        uint32_t v = 0;
-        if (i < end) {
-          v = index[i];
-          const float4 l = plo[job.prim_offset + v], h = phi[job.prim_offset + v];
-          const float c = 0.5f * ((&l.x)[axis] + (&h.x)[axis]);
-          const int b = min(kSahBins - 1, max(0, (int)((c - cmin[axis]) * scale[axis])));
-          goes_left = b <= split ? 1u : 0u;
-        }
-        uint32_t prefix, tile_total;
-        BlockScan(scan_storage).ExclusiveSum(goes_left, prefix, tile_total);
-        __syncthreads();
-        if (i < end) {
-          if (goes_left) tmp[begin + left_base + prefix] = v;
-          else tmp[begin + (count - 1) - ((i - begin) - (left_base + prefix))] = v;
-        }
-        left_base += tile_total;
-        left_total = left_base;
-      }
-      __syncthreads();
-      // Rights were written back to front; copy both halves in order.
-      for (uint32_t i = begin + tid; i < end; i += blockDim.x) {
-        const uint32_t k = i - begin;
-        index[i] = k < left_total ? tmp[i] : tmp[begin + (count - 1) - (k - left_total)];
-      }
-      mid = begin + left_total;
-      if (mid == begin || mid == end) mid = begin + count / 2;
+      if (sp == 0) return;
+      --sp;
+      begin = stack[sp][0];
+      end = stack[sp][1];
+      slot = stack[sp][2];
     }
     __syncthreads();
-    // Children bounds: a reduction over each half.
-    if (tid < 6) sh.nb[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;
-    if (tid < 6) sh.cb[tid] = tid < 3 ? 0xFFFFFFFFu : 0u;  // reused for the right child
-    __syncthreads();
-    for (uint32_t i = begin + tid; i < end; i += blockDim.x) {
-      const float4 l = plo[job.prim_offset + index[i]], h = phi[job.prim_offset + index[i]];
-      uint32_t* b = i < mid ? sh.nb : sh.cb;
-      atomicMin(&b[0], ordered(l.x)); atomicMin(&b[1], ordered(l.y)); atomicMin(&b[2], ordered(l.z));
-      atomicMax(&b[3], ordered(h.x)); atomicMax(&b[4], ordered(h.y)); atomicMax(&b[5], ordered(h.z));
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const uint32_t ranges[2][2] = {{begin, mid}, {mid, end}};
-      const uint32_t* bounds[2] = {sh.nb, sh.cb};
-      int32_t child[2], ccount[2];
-      for (int k = 0; k < 2; ++k) {
-        const uint32_t n = ranges[k][1] - ranges[k][0];
-        if (n <= job.leaf_size) {
-          child[k] = job.leaves_are_values ? ~(int32_t)index[ranges[k][0]]
-                                           : ~(int32_t)(job.leaf_base + ranges[k][0]);
-          ccount[k] = (int32_t)n;
-        } else {
-          const uint32_t slot = sh.next_node++;
-          if (sh.sp >= kSahStack || slot >= job.count) {
-            sh.error = 1;
-            child[k] = kEmptyChild;
-            ccount[k] = 0;
-            continue;
-          }
-          sh.stack_begin[sh.sp] = ranges[k][0];
-          sh.stack_end[sh.sp] = ranges[k][1];
-          sh.stack_node[sh.sp] = slot;
-          ++sh.sp;
-          child[k] = (int32_t)(job.node_base + slot);
-          ccount[k] = 0;
-        }
+  }
+}
+
+constexpr int kMediumWarps = 4;
+__global__ void __launch_bounds__(32 * kMediumWarps) k_sah_medium(const SahJob* __restrict__ jobs,
+    const float4* __restrict__ plo, const float4* __restrict__ phi, uint32_t* __restrict__ idx,
+    uint32_t* __restrict__ scratch, BvhNode* __restrict__ nodes, SahLists lists) {
+  __shared__ SahShared<32> shared[kMediumWarps];
+  __shared__ uint32_t stacks[kMediumWarps][16][3];
+  SahShared<32>& sh = shared[threadIdx.x >> 5];
+  uint32_t(*stack)[3] = stacks[threadIdx.x >> 5];
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t total = lists.counters[kMediumCount];
+  for (;;) {
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&lists.counters[kMediumTaken], 1u);
+    at = __shfl_sync(kAllLanes, at, 0);
+    if (at >= total) return;
+    const SahNode root = lists.medium[at];
+    const SahJob job = jobs[root.job];
+    uint32_t begin = root.begin, end = root.end, slot = root.slot;
+    int sp = 0;
+    for (uint32_t step = 0; step < kSahMedium; ++step) {
+      const uint32_t mid = sah_split<32>(job, begin, end, slot, plo, phi, idx + job.prim_offset,
+          scratch + job.prim_offset, nodes, sh);
+      uint32_t r[2][3] = {{begin, mid, slot + 1}, {mid, end, slot + (mid - begin)}};
+      const bool keep[2] = {sah_keep(job, root.job, r[0][0], r[0][1], r[0][2], kSahSmall, lists, lane == 0),
+          sah_keep(job, root.job, r[1][0], r[1][1], r[1][2], kSahSmall, lists, lane == 0)};
+      int next = keep[0] ? 0 : keep[1] ? 1 : -1;
+      if (keep[0] && keep[1]) {
+        // The smaller side first: at most one range per halving of kSahMedium.
+        next = mid - begin <= end - mid ? 0 : 1;
+        if (lane < 3) stack[sp][lane] = next ? r[0][lane] : r[1][lane];
+        ++sp;
       }
-      BvhNode nd;
-      nd.x = make_float4(unordered(bounds[0][0]), unordered(bounds[0][3]), unordered(bounds[1][0]), unordered(bounds[1][3]));
-      nd.y = make_float4(unordered(bounds[0][1]), unordered(bounds[0][4]), unordered(bounds[1][1]), unordered(bounds[1][4]));
-      nd.z = make_float4(unordered(bounds[0][2]), unordered(bounds[0][5]), unordered(bounds[1][2]), unordered(bounds[1][5]));
-      nd.c = make_int4(child[0], child[1], ccount[0], ccount[1]);
-      nodes[job.node_base + sh.node] = nd;
+      __syncwarp();
+      if (next >= 0) {
+        begin = next ? r[1][0] : r[0][0];
+        end = next ? r[1][1] : r[0][1];
+        slot = next ? r[1][2] : r[0][2];
+      } else {
+        if (sp == 0) break;
+        --sp;
+        begin = stack[sp][0];
+        end = stack[sp][1];
+        slot = stack[sp][2];
+      }
+      __syncwarp();
     }
   }
-  __syncthreads();
-  if (tid == 0 && (sh.error || sh.sp != 0)) atomicAdd(errors, 1u);
+}
+
+// Subtrees of at most 32 primitives, one primitive a lane, level by level:
+// each lane of a node tries the split after its own centroid on each axis
+// (ties by lane), the node's cheapest is taken, and the primitives move to
+// their side in order. A level takes as many steps as its largest node has
+// primitives, whatever the number of nodes.
+constexpr int kSmallWarps = 8;
+__global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const SahJob* __restrict__ jobs,
+    const float4* __restrict__ plo, const float4* __restrict__ phi, uint32_t* __restrict__ idx,
+    BvhNode* __restrict__ nodes, SahLists lists) {
+  __shared__ float4 shared_lo[kSmallWarps][32], shared_hi[kSmallWarps][32];  // w of lo: the primitive
+  __shared__ float shared_keys[kSmallWarps][32];
+  __shared__ int shared_axes[kSmallWarps][32];
+  float4* lo = shared_lo[threadIdx.x >> 5];
+  float4* hi = shared_hi[threadIdx.x >> 5];
+  float* keys = shared_keys[threadIdx.x >> 5];
+  int* axes = shared_axes[threadIdx.x >> 5];
+  const unsigned lane = threadIdx.x & 31u;
+  const uint32_t total = lists.counters[kSmallCount];
+  for (;;) {
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&lists.counters[kSmallTaken], 1u);
+    at = __shfl_sync(kAllLanes, at, 0);
+    if (at >= total) return;
+    const SahNode root = lists.small[at];
+    const SahJob job = jobs[root.job];
+    const uint32_t n = root.end - root.begin;
+    uint32_t* index = idx + job.prim_offset + root.begin;
+    {
+      const uint32_t v = lane < n ? index[lane] : 0u;
+      float4 l = lane < n ? plo[job.prim_offset + v] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      l.w = __uint_as_float(v);
+      lo[lane] = l;
+      hi[lane] = lane < n ? phi[job.prim_offset + v] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    __syncwarp();
+    // This lane's node: lanes [begin, end), its slot.
+    uint32_t begin = lane < n ? 0u : lane, end = lane < n ? n : lane, slot = root.slot;
+    for (int level = 0; level < 32; ++level) {
+      const bool inner = end - begin > job.leaf_size;
+      if (!__any_sync(kAllLanes, inner)) break;
+      float cost = INFINITY, box[12];
+      int axis = 0;
+      if (inner) {
+        const float4 ml = lo[lane], mh = hi[lane];
+        const float c[3] = {ml.x + mh.x, ml.y + mh.y, ml.z + mh.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          float b[12];
+#pragma unroll
+          for (int k = 0; k < 12; ++k) b[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
+          uint32_t lefts = 0;
+          for (uint32_t j = begin; j < end; ++j) {
+            const float4 l = lo[j], h = hi[j];
+            const float cj = a == 0 ? l.x + h.x : a == 1 ? l.y + h.y : l.z + h.z;
+            if (cj < c[a] || (cj == c[a] && j <= lane)) {
+              ++lefts;
+              b[0] = fminf(b[0], l.x); b[1] = fminf(b[1], l.y); b[2] = fminf(b[2], l.z);
+              b[3] = fmaxf(b[3], h.x); b[4] = fmaxf(b[4], h.y); b[5] = fmaxf(b[5], h.z);
+            } else {
+              b[6] = fminf(b[6], l.x); b[7] = fminf(b[7], l.y); b[8] = fminf(b[8], l.z);
+              b[9] = fmaxf(b[9], h.x); b[10] = fmaxf(b[10], h.y); b[11] = fmaxf(b[11], h.z);
+            }
+          }
+          const uint32_t rights = end - begin - lefts;
+          if (rights == 0) continue;
+          const float v = sah_half_area(b, b + 3) * (float)lefts + sah_half_area(b + 6, b + 9) * (float)rights;
+          if (v < cost) {
+            cost = v;
+            axis = a;
+#pragma unroll
+            for (int k = 0; k < 12; ++k) box[k] = b[k];
+          }
+        }
+      }
+      keys[lane] = cost;
+      axes[lane] = axis;
+      __syncwarp();
+      // The node's cheapest split (the first of equals); the middle of its
+      // lanes where no cost is finite (boxes beyond the floats' range).
+      unsigned pivot = lane;
+      int by = 3;
+      if (inner) {
+        float best = INFINITY;
+        for (uint32_t j = begin; j < end; ++j)
+          if (keys[j] < best) {
+            best = keys[j];
+            pivot = j;
+          }
+        if (best < INFINITY) {
+          by = axes[pivot];
+        } else {
+          pivot = begin + (end - begin) / 2 - 1;
+          if (lane == pivot) {
+#pragma unroll
+            for (int k = 0; k < 12; ++k) box[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
+            for (uint32_t j = begin; j < end; ++j) {
+              const float4 l = lo[j], h = hi[j];
+              if (j <= pivot) {
+                box[0] = fminf(box[0], l.x); box[1] = fminf(box[1], l.y); box[2] = fminf(box[2], l.z);
+                box[3] = fmaxf(box[3], h.x); box[4] = fmaxf(box[4], h.y); box[5] = fmaxf(box[5], h.z);
+              } else {
+                box[6] = fminf(box[6], l.x); box[7] = fminf(box[7], l.y); box[8] = fminf(box[8], l.z);
+                box[9] = fmaxf(box[9], h.x); box[10] = fmaxf(box[10], h.y); box[11] = fmaxf(box[11], h.z);
+              }
+            }
+          }
+        }
+      }
+      const float4 ml = lo[lane], mh = hi[lane], pl = lo[pivot], ph = hi[pivot];
+      const float mine = by == 0 ? ml.x + mh.x : by == 1 ? ml.y + mh.y : ml.z + mh.z;
+      const float at_pivot = by == 0 ? pl.x + ph.x : by == 1 ? pl.y + ph.y : pl.z + ph.z;
+      const bool left = by == 3 ? lane <= pivot : mine < at_pivot || (mine == at_pivot && lane <= pivot);
+      const unsigned lefts = __ballot_sync(kAllLanes, left);
+      const unsigned in_node = end - begin == 32u ? kAllLanes : ((1u << (end - begin)) - 1u) << (begin & 31u);
+      const unsigned below = (1u << lane) - 1u;
+      const uint32_t mid = begin + (uint32_t)__popc(lefts & in_node);
+      const uint32_t to = !inner ? lane
+          : left ? begin + (uint32_t)__popc(lefts & in_node & below) : mid + (uint32_t)__popc(~lefts & in_node & below);
+      __syncwarp();
+      lo[to] = ml;
+      hi[to] = mh;
+      __syncwarp();
+      if (inner && lane == pivot) {
+        auto child = [&](uint32_t first, uint32_t last, uint32_t child_slot, int32_t& count) {
+          count = last - first <= job.leaf_size ? (int32_t)(last - first) : 0;
+          if (count == 0) return (int32_t)(job.node_base + child_slot);
+          return job.leaves_are_values ? ~(int32_t)__float_as_uint(lo[first].w)
+                                       : ~(int32_t)(job.leaf_base + root.begin + first);
+        };
+        int32_t n0, n1;
+        const int32_t c0 = child(begin, mid, slot + 1, n0), c1 = child(mid, end, slot + (mid - begin), n1);
+        BvhNode nd;
+        nd.x = make_float4(box[0], box[3], box[6], box[9]);
+        nd.y = make_float4(box[1], box[4], box[7], box[10]);
+        nd.z = make_float4(box[2], box[5], box[8], box[11]);
+        nd.c = make_int4(c0, c1, n0, n1);
+        nodes[job.node_base + slot] = nd;
+      }
+      // This lane's node from here on is the half it lies in.
+      if (inner) {
+        if (lane < mid) {
+          end = mid;
+          slot += 1;
+        } else {
+          slot += mid - begin;
+          begin = mid;
+        }
+      }
+      __syncwarp();
+    }
+    if (lane < n) index[lane] = __float_as_uint(lo[lane].w);
+    __syncwarp();
+  }
+}
+
+// The job that holds primitive g of the batch (jobs in order of prim_offset).
+__device__ __forceinline__ uint32_t sah_job_of(const SahJob* __restrict__ jobs, uint32_t count, uint32_t g) {
+  uint32_t lo = 0, hi = count;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (jobs[mid].prim_offset <= g) lo = mid;
+    else hi = mid;
+  }
+  return lo;
 }
 
 // Triangle boxes of every geometry of a batch: primitive i of job j at
 // prim_offset + i, its positions and triangles at the job's offsets.
 __global__ void k_batch_triangle_boxes(const float* __restrict__ positions, const uint32_t* __restrict__ triangles,
-    const uint64_t* __restrict__ vbase, const uint32_t* __restrict__ prim_job, const SahJob* __restrict__ jobs,
-    uint32_t total, float4* __restrict__ lo, float4* __restrict__ hi, uint32_t* __restrict__ idx) {
+    const SahJob* __restrict__ jobs, uint32_t job_count, uint32_t total, float4* __restrict__ lo,
+    float4* __restrict__ hi, uint32_t* __restrict__ idx) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
-  const uint32_t j = prim_job[g];
-  const uint32_t local = g - jobs[j].prim_offset;
-  const float* P = positions + 3 * vbase[j];
+  const SahJob& job = jobs[sah_job_of(jobs, job_count, g)];
+  const uint32_t local = g - job.prim_offset;
+  const float* P = positions + 3 * job.vertex_offset;
+  const uint32_t* T = triangles + 3 * (job.triangle_offset + local);
   float l[3] = {kFloatMax, kFloatMax, kFloatMax}, h[3] = {-kFloatMax, -kFloatMax, -kFloatMax};
   for (int k = 0; k < 3; ++k) {
-    const uint32_t v = triangles[3 * (size_t)g + k];
+    const uint32_t v = T[k];
     for (int a = 0; a < 3; ++a) {
       const float p = P[3 * (size_t)v + a];
       l[a] = fminf(l[a], p);
@@ -582,19 +882,18 @@ __global__ void k_batch_triangle_boxes(const float* __restrict__ positions, cons
 // The leaf-ordered triangle pool of a batch: pool slot leaf_base + i holds
 // triangle idx[prim_offset + i] of job j.
 __global__ void k_batch_write_triangles(const float* __restrict__ positions, const uint32_t* __restrict__ triangles,
-    const uint64_t* __restrict__ vbase, const uint64_t* __restrict__ tbase, const uint32_t* __restrict__ prim_job,
-    const SahJob* __restrict__ jobs, const uint32_t* __restrict__ idx, uint32_t total, float4* __restrict__ pool) {
+    const SahJob* __restrict__ jobs, uint32_t job_count, const uint32_t* __restrict__ idx, uint32_t total,
+    float4* __restrict__ pool) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= total) return;
-  const uint32_t j = prim_job[g];
-  const SahJob job = jobs[j];
+  const SahJob& job = jobs[sah_job_of(jobs, job_count, g)];
   const uint32_t local = g - job.prim_offset;
   const uint32_t p = idx[g];
-  const float* P = positions + 3 * vbase[j];
-  const uint32_t* T = triangles + 3 * tbase[j];
+  const float* P = positions + 3 * job.vertex_offset;
+  const uint32_t* T = triangles + 3 * (job.triangle_offset + p);
   float4* out = pool + kTriStride * (size_t)(job.leaf_base + local);
   for (int k = 0; k < 3; ++k) {
-    const uint32_t v = T[3 * (size_t)p + k];
+    const uint32_t v = T[k];
     out[k] = make_float4(P[3 * (size_t)v], P[3 * (size_t)v + 1], P[3 * (size_t)v + 2],
         k == 0 ? __uint_as_float(p) : 0.0f);
   }
@@ -708,8 +1007,9 @@ __global__ void k_refit_parents(const BvhNode* __restrict__ nodes, uint32_t node
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const int4 c = nodes[node_base + i].c;
-  if (c.x >= 0 && c.x != kEmptyChild) parent[(uint32_t)c.x - node_base] = node_base + i;
-  if (c.y >= 0 && c.y != kEmptyChild) parent[(uint32_t)c.y - node_base] = node_base + i;
+  // Slots that a tree with larger leaves leaves unused name no node of it.
+  if (c.x >= 0 && (uint32_t)c.x - node_base < count) parent[(uint32_t)c.x - node_base] = node_base + i;
+  if (c.y >= 0 && (uint32_t)c.y - node_base < count) parent[(uint32_t)c.y - node_base] = node_base + i;
   arrivals[i] = 0;
 }
 
@@ -777,6 +1077,9 @@ __global__ void k_refit_up(BvhNode* nodes, const float4* __restrict__ pool, uint
   }
 }
 
+// Blocks of the SAH list kernels: up to eight on each of a B200's SMs.
+constexpr uint32_t kListBlocks = 148 * 8;
+
 inline uint32_t blocks(uint64_t n) { return (uint32_t)((n + kBuildBlock - 1) / kBuildBlock); }
 
 }  // namespace
@@ -809,7 +1112,7 @@ cudaError_t BvhBuilder::reserve(uint32_t n, cudaStream_t stream) {
       !alloc((void**)&nlo_, nn * 16) || !alloc((void**)&nhi_, nn * 16) ||
       !alloc((void**)&left_, nn * 4) || !alloc((void**)&right_, nn * 4) ||
       !alloc((void**)&parent_internal_, nn * 4) || !alloc((void**)&parent_leaf_, nn * 4) ||
-      !alloc((void**)&flags_, nn * 4) || !alloc((void**)&bounds_, 6 * 4))
+      !alloc((void**)&flags_, nn * 4) || !alloc((void**)&bounds_, (8 + kSahCounters) * 4))
     return e;
   size_t temp = 0;
   cub::DoubleBuffer<uint64_t> k(keys_, keys_alt_);
@@ -823,7 +1126,7 @@ cudaError_t BvhBuilder::reserve(uint32_t n, cudaStream_t stream) {
 
 void BvhBuilder::release() {
   void* ptrs[] = {keys_, keys_alt_, values_, values_alt_, plo_, phi_, nlo_, nhi_, left_, right_,
-      parent_internal_, parent_leaf_, flags_, bounds_, temp_};
+      parent_internal_, parent_leaf_, flags_, bounds_, temp_, jobs_};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   keys_ = keys_alt_ = nullptr;
@@ -831,6 +1134,8 @@ void BvhBuilder::release() {
   plo_ = phi_ = nlo_ = nhi_ = nullptr;
   left_ = right_ = parent_internal_ = parent_leaf_ = flags_ = bounds_ = nullptr;
   temp_ = nullptr;
+  jobs_ = nullptr;
+  job_capacity_ = 0;
   capacity_ = 0;
   temp_bytes_ = 0;
 }
@@ -879,97 +1184,84 @@ cudaError_t BvhBuilder::build_triangles(const float* positions, const uint32_t* 
   return cudaGetLastError();
 }
 
+// Builds the jobs' trees over the boxes in plo_ / phi_ and the indices in
+// values_ (both in batch order). One word of errors is left for the caller
+// to read.
+cudaError_t BvhBuilder::sah_build(const std::vector<SahJob>& jobs, uint32_t total, BvhNode* nodes,
+    cudaStream_t stream) {
+  uint32_t largest = 0;
+  for (const SahJob& j : jobs) {
+    largest = std::max(largest, j.count);
+    // Leaves of several triangles leave node slots unused, which the refit
+    // and the collapse read: as references to no node.
+    if (j.leaf_size > 1) cudaMemsetAsync(nodes + j.node_base, 0x7F, node_count(j.count) * sizeof(BvhNode), stream);
+  }
+  SahLists lists{reinterpret_cast<SahNode*>(keys_alt_), reinterpret_cast<SahNode*>(keys_), bounds_ + 8};
+  cudaMemsetAsync(lists.counters, 0, kSahCounters * sizeof(uint32_t), stream);
+  k_sah_large<<<(uint32_t)jobs.size(), kSahBlock, 0, stream>>>(jobs_, plo_, phi_, values_, values_alt_, nodes, lists);
+  if (largest > kSahSmall) {
+    const uint32_t grid = std::min(kListBlocks, total / (kSahSmall * kMediumWarps) + 1);
+    k_sah_medium<<<grid, 32 * kMediumWarps, 0, stream>>>(jobs_, plo_, phi_, values_, values_alt_, nodes, lists);
+  }
+  if (largest > 1) {
+    const uint32_t grid = std::min(kListBlocks, total / (2 * kSmallWarps) + 1);
+    k_sah_small<<<grid, 32 * kSmallWarps, 0, stream>>>(jobs_, plo_, phi_, values_, nodes, lists);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t BvhBuilder::upload_jobs(const std::vector<SahJob>& jobs, cudaStream_t stream) {
+  if (jobs.size() > job_capacity_) {
+    if (jobs_) cudaFree(jobs_);
+    jobs_ = nullptr;
+    job_capacity_ = 0;
+    const cudaError_t e = cudaMalloc(&jobs_, jobs.size() * sizeof(SahJob));
+    if (e != cudaSuccess) return e;
+    job_capacity_ = jobs.size();
+  }
+  return cudaMemcpyAsync(jobs_, jobs.data(), jobs.size() * sizeof(SahJob), cudaMemcpyHostToDevice, stream);
+}
+
+cudaError_t BvhBuilder::sah_errors(cudaStream_t stream) {
+  uint32_t errors = 0;
+  cudaMemcpyAsync(&errors, bounds_ + 8 + kSahErrors, 4, cudaMemcpyDeviceToHost, stream);
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return e;
+  return errors ? cudaErrorUnknown : cudaSuccess;
+}
+
 cudaError_t BvhBuilder::build_triangle_batch(const float* positions, const uint32_t* triangles,
     const std::vector<BatchGeometry>& geometries, BvhNode* nodes, float4* tri_pool, cudaStream_t stream,
     uint32_t leaf_size) {
   std::vector<SahJob> jobs;
-  std::vector<uint64_t> vbase, tbase;
   uint32_t total = 0;
   for (const BatchGeometry& g : geometries) {
     if (g.count == 0) continue;
-    SahJob j;
-    j.prim_offset = total;
-    j.count = g.count;
-    j.node_base = g.node_base;
-    j.leaf_base = g.tri_base;
-    j.leaf_size = leaf_size;
-    j.leaves_are_values = 0;
-    jobs.push_back(j);
-    vbase.push_back(g.vertex_offset);
-    tbase.push_back(g.tri_base);
+    jobs.push_back(SahJob{total, g.count, g.node_base, g.tri_base, leaf_size, 0, g.vertex_offset, g.tri_base});
     total += g.count;
   }
   if (jobs.empty()) return cudaSuccess;
-  std::vector<uint32_t> prim_job(total);
-  for (uint32_t k = 0; k < jobs.size(); ++k)
-    for (uint32_t i = 0; i < jobs[k].count; ++i) prim_job[jobs[k].prim_offset + i] = k;
   cudaError_t e = reserve(total, stream);
-  if (e != cudaSuccess) return e;
-  SahJob* d_jobs = nullptr;
-  uint64_t* d_vbase = nullptr;
-  uint64_t* d_tbase = nullptr;
-  uint32_t* d_prim_job = nullptr;
-  uint32_t* d_tris = nullptr;
-  if ((e = cudaMalloc(&d_jobs, jobs.size() * sizeof(SahJob))) != cudaSuccess ||
-      (e = cudaMalloc(&d_vbase, jobs.size() * 8)) != cudaSuccess ||
-      (e = cudaMalloc(&d_tbase, jobs.size() * 8)) != cudaSuccess ||
-      (e = cudaMalloc(&d_prim_job, (size_t)total * 4)) != cudaSuccess ||
-      (e = cudaMalloc(&d_tris, (size_t)total * 12)) != cudaSuccess)
-    return e;
-  cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(SahJob), cudaMemcpyHostToDevice, stream);
-  cudaMemcpyAsync(d_vbase, vbase.data(), jobs.size() * 8, cudaMemcpyHostToDevice, stream);
-  cudaMemcpyAsync(d_tbase, tbase.data(), jobs.size() * 8, cudaMemcpyHostToDevice, stream);
-  cudaMemcpyAsync(d_prim_job, prim_job.data(), (size_t)total * 4, cudaMemcpyHostToDevice, stream);
-  // Each job's triangles, gathered in batch order.
-  for (size_t k = 0; k < jobs.size(); ++k)
-    cudaMemcpyAsync(d_tris + 3 * (size_t)jobs[k].prim_offset, triangles + 3 * tbase[k], (size_t)jobs[k].count * 12,
-        cudaMemcpyDeviceToDevice, stream);
-  k_batch_triangle_boxes<<<blocks(total), kBuildBlock, 0, stream>>>(positions, d_tris, d_vbase, d_prim_job,
-      d_jobs, total, plo_, phi_, values_);
-  cudaMemsetAsync(flags_, 0, 4, stream);
-  k_sah_build<<<(uint32_t)jobs.size(), kSahBlock, 0, stream>>>(d_jobs, plo_, phi_, values_, values_alt_, nodes,
-      flags_);
-  // The pool: leaf_base is the geometry's tri_base, and the batch's
-  // triangles are addressed through the gathered copy.
-  std::vector<uint64_t> zero(jobs.size());
-  for (size_t k = 0; k < jobs.size(); ++k) zero[k] = jobs[k].prim_offset;
-  cudaMemcpyAsync(d_tbase, zero.data(), jobs.size() * 8, cudaMemcpyHostToDevice, stream);
-  k_batch_write_triangles<<<blocks(total), kBuildBlock, 0, stream>>>(positions, d_tris, d_vbase, d_tbase,
-      d_prim_job, d_jobs, values_, total, tri_pool);
-  uint32_t errors = 0;
-  cudaMemcpyAsync(&errors, flags_, 4, cudaMemcpyDeviceToHost, stream);
-  e = cudaStreamSynchronize(stream);
-  cudaFree(d_jobs);
-  cudaFree(d_vbase);
-  cudaFree(d_tbase);
-  cudaFree(d_prim_job);
-  cudaFree(d_tris);
-  if (e != cudaSuccess) return e;
-  return errors ? cudaErrorUnknown : cudaSuccess;
+  if (e != cudaSuccess || (e = upload_jobs(jobs, stream)) != cudaSuccess) return e;
+  const uint32_t count = (uint32_t)jobs.size();
+  k_batch_triangle_boxes<<<blocks(total), kBuildBlock, 0, stream>>>(positions, triangles, jobs_, count, total, plo_,
+      phi_, values_);
+  if ((e = sah_build(jobs, total, nodes, stream)) != cudaSuccess) return e;
+  k_batch_write_triangles<<<blocks(total), kBuildBlock, 0, stream>>>(positions, triangles, jobs_, count, values_,
+      total, tri_pool);
+  return sah_errors(stream);
 }
 
 cudaError_t BvhBuilder::build_instances_sah(const InstanceShading* shade, const InstanceTraversal* trav,
     const BvhNode* blas, uint32_t n, BvhNode* nodes, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
+  const std::vector<SahJob> jobs(1, SahJob{0, n, 0, 0, 1, 1, 0, 0});
   cudaError_t e = reserve(n, stream);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || (e = upload_jobs(jobs, stream)) != cudaSuccess) return e;
   init_bounds(bounds_, stream);
-  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, bounds_);
-  std::vector<uint32_t> iota(n);
-  for (uint32_t i = 0; i < n; ++i) iota[i] = i;
-  cudaMemcpyAsync(values_, iota.data(), (size_t)n * 4, cudaMemcpyHostToDevice, stream);
-  SahJob job{0, n, 0, 0, 1, 1};
-  SahJob* d_job = nullptr;
-  if ((e = cudaMalloc(&d_job, sizeof(SahJob))) != cudaSuccess) return e;
-  cudaMemcpyAsync(d_job, &job, sizeof(job), cudaMemcpyHostToDevice, stream);
-  cudaMemsetAsync(flags_, 0, 4, stream);
-  k_sah_build<<<1, kSahBlock, 0, stream>>>(d_job, plo_, phi_, values_, values_alt_, nodes, flags_);
-  uint32_t errors = 0;
-  cudaMemcpyAsync(&errors, flags_, 4, cudaMemcpyDeviceToHost, stream);
-  e = cudaStreamSynchronize(stream);
-  cudaFree(d_job);
-  if (e != cudaSuccess) return e;
-  return errors ? cudaErrorUnknown : cudaSuccess;
+  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, bounds_, values_);
+  if ((e = sah_build(jobs, n, nodes, stream)) != cudaSuccess) return e;
+  return sah_errors(stream);
 }
 
 cudaError_t BvhBuilder::collapse(const BvhNode* binary, uint32_t n, Bvh4Node* wide, bool leaves_are_instances,
@@ -992,7 +1284,7 @@ cudaError_t BvhBuilder::build_instances(const InstanceShading* shade,
   cudaError_t e = reserve(n, stream);
   if (e != cudaSuccess) return e;
   init_bounds(bounds_, stream);
-  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, bounds_);
+  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, bounds_, nullptr);
   const uint32_t* sorted = nullptr;
   return build_common(n, nodes, 0, 0, true, stream, &sorted);
 }

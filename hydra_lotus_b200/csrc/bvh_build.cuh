@@ -1,5 +1,5 @@
 // SPDX-License-Identifier: Apache-2.0
-// On-device BVH builders: per-CTA binned SAH and LBVH (see bvh_build.cu).
+// On-device BVH builders: batched SAH and LBVH (see bvh_build.cu).
 #pragma once
 
 #include <vector>
@@ -17,19 +17,31 @@ struct BatchGeometry {
   uint32_t node_base;
 };
 
-// Geometries up to this many triangles build with the per-CTA binned-SAH
-// builder; larger ones with the LBVH.
+// One BVH of a batch of SAH builds.
+struct SahJob {
+  uint32_t prim_offset;  // first primitive in the batch's arrays
+  uint32_t count;
+  uint32_t node_base;    // first node slot
+  uint32_t leaf_base;    // first triangle-pool slot (BLAS)
+  uint32_t leaf_size;    // most primitives per leaf
+  uint32_t leaves_are_values;  // TLAS: leaves hold the primitive index itself
+  uint64_t vertex_offset;      // BLAS: first vertex and triangle
+  uint64_t triangle_offset;
+};
+
+// Geometries up to this many triangles build with the SAH builder; larger
+// ones with the LBVH.
 constexpr uint32_t kSahMaxTriangles = 65536;
 
 // Scratch for building BVHs, grown to the largest primitive count seen. A
 // BVH over n > 1 primitives has at most n - 1 nodes; over one, one.
 class BvhBuilder {
  public:
-  // Binned-SAH BLASes of many geometries in one launch (one CTA each).
+  // SAH BLASes of many geometries together.
   cudaError_t build_triangle_batch(const float* positions, const uint32_t* triangles,
       const std::vector<BatchGeometry>& geometries, BvhNode* nodes, float4* tri_pool, cudaStream_t stream,
       uint32_t leaf_size);
-  // The binned-SAH TLAS (one instance per leaf).
+  // The SAH TLAS (one instance per leaf).
   cudaError_t build_instances_sah(const InstanceShading* shade, const InstanceTraversal* trav,
       const BvhNode* blas, uint32_t n, BvhNode* nodes, cudaStream_t stream);
   ~BvhBuilder() { release(); }
@@ -60,6 +72,9 @@ class BvhBuilder {
   static uint32_t node_count(uint32_t n) { return n > 1 ? n - 1 : n; }
 
  private:
+  cudaError_t sah_build(const std::vector<SahJob>& jobs, uint32_t total, BvhNode* nodes, cudaStream_t stream);
+  cudaError_t upload_jobs(const std::vector<SahJob>& jobs, cudaStream_t stream);
+  cudaError_t sah_errors(cudaStream_t stream);
   cudaError_t reserve(uint32_t n, cudaStream_t stream);
   cudaError_t build_common(uint32_t n, BvhNode* nodes, uint32_t node_base, uint32_t leaf_base,
       bool leaves_are_values, cudaStream_t stream, const uint32_t** sorted);
@@ -81,6 +96,8 @@ class BvhBuilder {
   uint32_t* flags_ = nullptr;
   uint32_t* bounds_ = nullptr;
   void* temp_ = nullptr;
+  SahJob* jobs_ = nullptr;
+  size_t job_capacity_ = 0;
 };
 
 }  // namespace lotus
