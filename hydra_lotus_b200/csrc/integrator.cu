@@ -524,13 +524,34 @@ __global__ void __launch_bounds__(kBlock) k_wf_camera(SceneView S,
 // throughput and radiance so far and carry on.
 // kCacheVertex: the cache's vertex (bounce 1 with the cache enabled); the
 // other instantiation carries none of the cache's code or registers.
-// Compiled for six resident blocks per SM (80 registers): shading is
-// latency-bound and gains more from occupancy than from registers. The
-// full-shading instantiation (texture lookups, glTF PBR) at four (128
-// registers): at 80 it spilled 350-550 bytes a thread.
-constexpr int kShadeBlocksPerSm = 6;
+// Shading is bound by latency, memory's and the instruction cache's: its
+// code is larger than an SM's instruction cache (10% of the fetches miss),
+// and warps at different places of it evict one another's (a stall of 8
+// cycles an instruction at the sphere field's first bounce). A block
+// therefore starts each stride of its hits together. Shapes, with the
+// shading time of a case before and after:
+// - no analytic lights, no full shading: two blocks of 384 (80 registers).
+//   16 samples of the sphere field at 1280x720 5.90 -> 4.88 ms, 16 rooms of
+//   a batch 23.0 -> 20.1 (128 threads without starting together before). Three
+//   of 256: 4.91 and 20.4; one of 768: 4.76 and 18.7, but the box room at
+//   256 squared 1.60 -> 1.72, its launches too short for blocks that large;
+//   one of 512 without spills (118 registers): 5.41 and 21.2.
+// - analytic lights: six of 128 (larger ones 3 to 5% slower).
+// - full shading (texture lookups, glTF PBR): four of 128 (128 registers),
+//   glTF Cornell box at 1024 squared 0.85 -> 0.80 ms; two of 256 0.82, one of
+//   384 without spills 0.86.
+// - both: one of 384 (168 registers), texture fixture 1.96 -> 1.68 ms; one of
+//   512 or two of 256 at 128 registers 1.85.
+struct ShadeShape {
+  int threads, blocks_per_sm;
+};
+constexpr ShadeShape shade_shape(bool analytic, bool full_shading) {
+  if (full_shading) return analytic ? ShadeShape{384, 1} : ShadeShape{128, 4};
+  return analytic ? ShadeShape{128, 6} : ShadeShape{384, 2};
+}
 template <bool kCacheVertex, bool kBatch, bool kAnalytic, bool kFullShading>
-__global__ void __launch_bounds__(kBlock, kFullShading ? 4 : kShadeBlocksPerSm) k_wf_shade(SceneView S,
+__global__ void __launch_bounds__(shade_shape(kAnalytic, kFullShading).threads,
+    shade_shape(kAnalytic, kFullShading).blocks_per_sm) k_wf_shade(SceneView S,
     const FrameConst* __restrict__ fcp, PathState P, Queues Q, uint32_t bounce, CacheQueues C, SceneTable B) {
   const uint32_t n = Q.counts[3 * bounce + 1];
   const bool cache_vertex = kCacheVertex && bounce < fcp->max_bounces;
@@ -548,6 +569,7 @@ __global__ void __launch_bounds__(kBlock, kFullShading ? 4 : kShadeBlocksPerSm) 
   // the SMs, not to the largest queue, so that the short queues of late
   // bounces cost little).
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    __syncthreads();  // the block's warps start together (see ShadeShape)
     const uint32_t index = base + threadIdx.x;
     const bool valid = index < n;
     bool cont = false, query = false, training = false;
@@ -1283,6 +1305,15 @@ uint32_t persistent_grid(const void* kernel, uint32_t capacity, const TraceTunin
   return std::max(1u, std::min(grid, (capacity + kBlock - 1) / kBlock));
 }
 
+// Blocks of the shading kernel: up to eight waves of resident blocks, grid-
+// striding over longer queues.
+uint32_t shade_grid(const ShadeShape& shape, uint32_t capacity) {
+  int sms = 0;
+  blocks_per_sm((const void*)k_wf_extend<false, false, false, false>, sms);
+  const uint32_t threads = (uint32_t)shape.threads;
+  return std::min((capacity + threads - 1) / threads, 8u * (uint32_t)(sms * shape.blocks_per_sm));
+}
+
 uint32_t choose_wavefront_rounds(const uint32_t* counts, uint32_t resident, uint32_t max_bounces, uint32_t samples,
     uint32_t counted) {
   constexpr uint32_t kTailQueue = 65536;
@@ -1332,10 +1363,8 @@ void launch_wavefront_sample(const SceneView& S, const FrameConst* fc, const uin
   const uint32_t grid_shadow = persistent_grid(
       count ? (const void*)k_wf_shadow<true, false, true> : (const void*)k_wf_shadow<false, false, false>, Q.capacity,
       tuning);
-  // Shading: up to eight waves of resident blocks, grid-striding over
-  // longer queues.
-  const uint32_t grid_shade = std::min((Q.capacity + kBlock - 1) / kBlock,
-      8u * persistent_grid((const void*)k_wf_shade<false, false, false, false>, Q.capacity, TraceTuning()));
+  const ShadeShape shade = shade_shape(analytic, full_shading);
+  const uint32_t grid_shade = shade_grid(shade, Q.capacity);
   {
     // One camera thread per pixel of each of the wave's samples.
     Timed t(profile, stream, 0);
@@ -1383,10 +1412,10 @@ void launch_wavefront_sample(const SceneView& S, const FrameConst* fc, const uin
       Timed t(profile, stream, 2);
       with_features(analytic, full_shading, [&](auto a, auto x) {
         if (cache_vertex)
-          k_wf_shade<true, false, decltype(a)::value, decltype(x)::value><<<grid_shade, kBlock, 0, stream>>>(S, fc, P,
+          k_wf_shade<true, false, decltype(a)::value, decltype(x)::value><<<grid_shade, shade.threads, 0, stream>>>(S, fc, P,
               QS, b, C, none);
         else
-          k_wf_shade<false, false, decltype(a)::value, decltype(x)::value><<<grid_shade, kBlock, 0, stream>>>(S, fc, P,
+          k_wf_shade<false, false, decltype(a)::value, decltype(x)::value><<<grid_shade, shade.threads, 0, stream>>>(S, fc, P,
               QS, b, C, none);
       });
     }
@@ -1505,8 +1534,8 @@ void launch_wavefront_batch(const SceneTable& B, uint32_t max_bounces, const Pat
   const uint32_t grid_slots = (B.total_slots + kBlock - 1) / kBlock;
   const uint32_t grid_extend = persistent_grid((const void*)k_wf_extend<false, true, false, false>, Q.capacity, tuning);
   const uint32_t grid_shadow = persistent_grid((const void*)k_wf_shadow<false, true, true>, Q.capacity, tuning);
-  const uint32_t grid_shade = std::min((Q.capacity + kBlock - 1) / kBlock,
-      8u * persistent_grid((const void*)k_wf_shade<false, true, false, false>, Q.capacity, TraceTuning()));
+  const ShadeShape shade = shade_shape(B.analytic, B.full_shading);
+  const uint32_t grid_shade = shade_grid(shade, Q.capacity);
   if (B.full_shading) k_wf_camera<false, true, true><<<grid_slots, kBlock, 0, stream>>>(none_view, no_frame, P, Q, nullptr, B);
   else k_wf_camera<false, true, false><<<grid_slots, kBlock, 0, stream>>>(none_view, no_frame, P, Q, nullptr, B);
   const uint32_t rounds = wavefront_rounds(max_bounces, false, tuning.rounds);
@@ -1529,7 +1558,7 @@ void launch_wavefront_batch(const SceneTable& B, uint32_t max_bounces, const Pat
     if (keyed && b + 1 < rounds) cudaMemsetAsync(Q.bins, 0, sizeof(uint32_t) * kSortBins, stream);
     else QS.keys = nullptr;
     with_features(B.analytic, B.full_shading, [&](auto a, auto x) {
-      k_wf_shade<false, true, decltype(a)::value, decltype(x)::value><<<grid_shade, kBlock, 0, stream>>>(none_view,
+      k_wf_shade<false, true, decltype(a)::value, decltype(x)::value><<<grid_shade, shade.threads, 0, stream>>>(none_view,
           B.frames, P, QS, b, no_cache, B);
     });
     if (B.full_shading)
