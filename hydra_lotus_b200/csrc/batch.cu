@@ -365,15 +365,13 @@ extern "C" int32_t lotus_cuda_batch_render(lotus_cuda_batch* b, const lotus_fram
   bool analytic = false, full_shading = false;
   // Every scene's walks report to the first scene's walk-failure words.
   uint32_t* walk_failure = nullptr;
-  uint32_t step_limit = 0;
+  uint32_t step_limit = kMaxTraversalSteps;
   for (uint32_t k = 0; k < count; ++k) {
     RendererAccess a;
     if (!renderer_access(b->scenes[k], a, detail)) return fail("scene " + std::to_string(k) + ": " + detail);
     views[k] = *a.view;
-    if (!walk_failure) {
-      walk_failure = a.view->walk_failure;
-      step_limit = a.step_limit;
-    }
+    if (!walk_failure) walk_failure = a.view->walk_failure;
+    step_limit = std::min(step_limit, a.step_limit);
     views[k].walk_failure = walk_failure;
     analytic = analytic || a.view->analytic_count != 0;
     full_shading = full_shading || a.view->full_shading != 0;
@@ -384,6 +382,7 @@ extern "C" int32_t lotus_cuda_batch_render(lotus_cuda_batch* b, const lotus_fram
   B.slot_base = b->slot_base;
   B.count = count;
   B.total_slots = base[count];
+  B.step_limit = step_limit;
   B.analytic = analytic;
   B.full_shading = full_shading;
   {

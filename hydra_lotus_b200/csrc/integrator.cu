@@ -770,7 +770,8 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_shadow(SceneVi
       ++rays;
     }
     if (!__any_sync(kFullWarp, active)) break;
-    if (walk_round<true, kCount, kFullShading>(kBatch ? B.views[scene] : S, W, store, stack, rng, active, &vc)) {
+    if (walk_round<true, kCount, kFullShading>(kBatch ? B.views[scene] : S, W, store, stack, rng,
+            kBatch ? B.step_limit : S.step_limit, active, &vc)) {
       active = false;
       const float tr = W.transmittance;
       if (tr > 0.0f) {
@@ -880,7 +881,7 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_visibility(SceneV
       active = true;
     }
     if (!__any_sync(kFullWarp, active)) break;
-    if (walk_round<true, false, kFullShading>(S, W, store, stack, rng, active, nullptr)) {
+    if (walk_round<true, false, kFullShading>(S, W, store, stack, rng, S.step_limit, active, nullptr)) {
       active = false;
       const float visibility = W.transmittance;
       const uint32_t slot = VQ.slot[index];
@@ -940,7 +941,8 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocksPerSm) k_wf_extend(SceneVi
     if (!__any_sync(kFullWarp, active)) break;
     bool emit = false;
     const SceneView& SS = kBatch ? B.views[scene] : S;
-    if (walk_round<false, kCount, kFullShading>(SS, W, store, stack, rng, active, &vc)) {
+    if (walk_round<false, kCount, kFullShading>(SS, W, store, stack, rng, kBatch ? B.step_limit : S.step_limit,
+            active, &vc)) {
       active = false;
       if (W.is(kWalkFound)) {
         P.hit[slot] = store.hit();

@@ -106,6 +106,7 @@ struct SceneTable {
   const uint32_t* slot_base = nullptr;  // count + 1 entries
   uint32_t count = 0;
   uint32_t total_slots = 0;
+  uint32_t step_limit = kMaxTraversalSteps;  // the smallest of the scenes' SceneView::step_limit
   bool analytic = false;  // some scene has analytic lights
   bool full_shading = false;  // some scene has texture lookups or glTF PBR materials
   // The camera pass's order within each scene: 0, each image's rows; k,
