@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -482,25 +483,15 @@ double world_triangle_area(const lotus_geometry& g, uint32_t t, const float* m) 
   return std::isfinite(area) ? area : 0.0;
 }
 
-double scene_radius(const lotus_scene_desc& s) {
+// `boxes`: each geometry's box (geometry_box).
+double scene_radius(const lotus_scene_desc& s, const std::vector<std::array<float, 6>>& boxes) {
   constexpr double kInf = std::numeric_limits<double>::infinity();
-  std::vector<std::array<double, 6>> object(s.geometry_count);
-  std::vector<char> done(s.geometry_count, 0);
   std::array<double, 6> world{kInf, kInf, kInf, -kInf, -kInf, -kInf};
   for (uint32_t i = 0; i < s.instance_count; ++i) {
     const lotus_instance& inst = s.instances[i];
-    auto& b = object[inst.geometry];
-    if (!done[inst.geometry]) {
-      done[inst.geometry] = 1;
-      b = {kInf, kInf, kInf, -kInf, -kInf, -kInf};
-      const lotus_geometry& g = s.geometries[inst.geometry];
-      for (uint32_t v = 0; v < g.vertex_count; ++v)
-        for (int a = 0; a < 3; ++a) {
-          b[a] = std::min(b[a], (double)g.positions[3 * (size_t)v + a]);
-          b[3 + a] = std::max(b[3 + a], (double)g.positions[3 * (size_t)v + a]);
-        }
-    }
-    if (!(b[0] <= b[3])) continue;
+    const std::array<float, 6>& f = boxes[inst.geometry];
+    if (!(f[0] <= f[3])) continue;
+    const double b[6] = {f[0], f[1], f[2], f[3], f[4], f[5]};
     const float* m = inst.world_from_object;
     for (int corner = 0; corner < 8; ++corner) {
       const double p[3] = {b[(corner & 1) ? 3 : 0], b[(corner & 2) ? 4 : 1], b[(corner & 4) ? 5 : 2]};
@@ -517,7 +508,8 @@ double scene_radius(const lotus_scene_desc& s) {
   return std::isfinite(radius) ? radius : 0.0;
 }
 
-LightTable build_light_table(const lotus_scene_desc& s, double env_mean) {
+LightTable build_light_table(const lotus_scene_desc& s, const std::vector<std::array<float, 6>>& boxes,
+    double env_mean) {
   LightTable table;
   table.offsets.assign(s.instance_count, kNoLights);
   std::vector<double> weights;
@@ -568,7 +560,7 @@ LightTable build_light_table(const lotus_scene_desc& s, double env_mean) {
   }
   bool distant = env_mean > 0.0;
   for (uint32_t i = 0; i < s.light_count; ++i) distant = distant || s.lights[i].shape == LOTUS_LIGHT_DISTANT;
-  const double r = distant ? scene_radius(s) : 0.0;
+  const double r = distant ? scene_radius(s, boxes) : 0.0;
   std::vector<uint32_t> analytic_entries;
   for (uint32_t i = 0; i < s.light_count; ++i) {
     double weight = 0.0;
@@ -657,9 +649,26 @@ constexpr uint64_t kWavePaths = 1ull << 21;
 // arrays (owned copies; `geometries` points into them), its box and its
 // places in the device arrays and pools, the materials and the
 // environment's summary.
+template <typename T>
+struct HostArena {
+  std::unique_ptr<T[]> data;
+  size_t capacity = 0;
+  // Uninitialised room for n elements; what it held is lost when it grows.
+  T* need(size_t n) {
+    if (n > capacity) {
+      data.reset(new T[n]);
+      capacity = n;
+    }
+    return data.get();
+  }
+};
+
 struct HostScene {
-  std::vector<std::vector<float>> positions, normals;
-  std::vector<std::vector<uint32_t>> triangles;
+  // Every geometry's positions and triangles, one after another (at its
+  // vertex_base and tri_base), as the device arrays hold them: one copy from
+  // the caller's arrays and one upload. A later scene reuses the room.
+  HostArena<float> positions;
+  HostArena<uint32_t> triangles;
   std::vector<lotus_geometry> geometries;
   std::vector<std::array<float, 6>> boxes;
   std::vector<uint64_t> vertex_base;
@@ -835,8 +844,10 @@ struct Renderer {
   uint32_t cache_generation = 0;  // bumped by every configuration
 
   // Captured CUDA graphs: a sample (wave and count 0), or a chain of `count`
-  // waves of `wave` samples. The least recently launched one is given up
-  // for a new one.
+  // waves of `wave` samples. The first launch of a key goes to the streams
+  // directly, the second is captured: a frame after a scene edit is often
+  // its key's only one, and capturing and instantiating takes longer than
+  // launching. The least recently launched one is given up for a new one.
   struct GraphKey {
     uint64_t scene_generation;
     uint32_t width, height, max_bounces;
@@ -851,6 +862,7 @@ struct Renderer {
     GraphKey key{};
     cudaGraphExec_t exec = nullptr;
     uint64_t used = 0;
+    bool seen = false;  // its key has been launched before
   };
   std::array<CapturedGraph, 8> graphs;
   uint64_t graph_clock = 0;
@@ -915,6 +927,18 @@ namespace {
 
 using namespace lotus;
 
+// Whether every value is finite, without a branch per value.
+bool all_finite(const float* values, uint64_t n) {
+  int32_t worst = 0;
+  for (uint64_t i = 0; i < n; ++i) {
+    int32_t bits;
+    std::memcpy(&bits, values + i, sizeof(bits));
+    bits &= 0x7FFFFFFF;
+    worst = bits > worst ? bits : worst;
+  }
+  return worst < 0x7F800000;
+}
+
 bool validate_scene(const lotus_scene_desc& s, std::string& detail) {
   if (s.material_count == 0 || !s.materials) {
     detail = "the scene has no material table";
@@ -971,21 +995,20 @@ bool validate_scene(const lotus_scene_desc& s, std::string& detail) {
       }
       color_values += geo.color_counts[k];
     }
-    for (uint64_t i = 0; i < 3 * color_values; ++i)
-      if (!std::isfinite(geo.colors[i])) {
-        detail = "geometry " + std::to_string(g) + " has a non-finite colour";
-        return false;
-      }
-    for (uint64_t i = 0; i < 3ull * geo.triangle_count; ++i)
-      if (geo.triangles[i] >= geo.vertex_count) {
-        detail = "geometry " + std::to_string(g) + " indexes past its vertices";
-        return false;
-      }
-    for (uint64_t i = 0; i < 3ull * geo.vertex_count; ++i)
-      if (!std::isfinite(geo.positions[i])) {
-        detail = "geometry " + std::to_string(g) + " has a non-finite position";
-        return false;
-      }
+    if (!all_finite(geo.colors, 3 * color_values)) {
+      detail = "geometry " + std::to_string(g) + " has a non-finite colour";
+      return false;
+    }
+    uint32_t past = 0;
+    for (uint64_t i = 0; i < 3ull * geo.triangle_count; ++i) past |= geo.triangles[i] >= geo.vertex_count ? 1u : 0u;
+    if (past) {
+      detail = "geometry " + std::to_string(g) + " indexes past its vertices";
+      return false;
+    }
+    if (!all_finite(geo.positions, 3ull * geo.vertex_count)) {
+      detail = "geometry " + std::to_string(g) + " has a non-finite position";
+      return false;
+    }
   }
   for (uint32_t i = 0; i < s.instance_count; ++i) {
     const lotus_instance& inst = s.instances[i];
@@ -1124,12 +1147,29 @@ lotus_scene_desc host_desc(const Renderer& R) {
 }
 
 std::array<float, 6> geometry_box(const lotus_geometry& geo) {
-  std::array<float, 6> b = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  for (uint32_t v = 0; v < geo.vertex_count; ++v)
-    for (int a = 0; a < 3; ++a) {
-      b[a] = std::min(b[a], geo.positions[3 * (size_t)v + a]);
-      b[3 + a] = std::max(b[3 + a], geo.positions[3 * (size_t)v + a]);
+  // Four vertices at a time: twelve running minima and maxima.
+  float lo[12], hi[12];
+  for (int k = 0; k < 12; ++k) {
+    lo[k] = INFINITY;
+    hi[k] = -INFINITY;
+  }
+  const float* p = geo.positions;
+  const uint64_t n = 3ull * geo.vertex_count, blocks = n / 12 * 12;
+  for (uint64_t i = 0; i < blocks; i += 12)
+    for (int k = 0; k < 12; ++k) {
+      lo[k] = p[i + k] < lo[k] ? p[i + k] : lo[k];
+      hi[k] = p[i + k] > hi[k] ? p[i + k] : hi[k];
     }
+  for (uint64_t i = blocks; i < n; ++i) {
+    const int k = (int)(i - blocks);
+    lo[k] = std::min(lo[k], p[i]);
+    hi[k] = std::max(hi[k], p[i]);
+  }
+  std::array<float, 6> b;
+  for (int a = 0; a < 3; ++a) {
+    b[a] = std::min(std::min(lo[a], lo[a + 3]), std::min(lo[a + 6], lo[a + 9]));
+    b[3 + a] = std::max(std::max(hi[a], hi[a + 3]), std::max(hi[a + 6], hi[a + 9]));
+  }
   return b;
 }
 
@@ -1137,7 +1177,7 @@ std::array<float, 6> geometry_box(const lotus_geometry& geo) {
 bool prepare_instances(Renderer& R, InstanceState& out, std::string& detail) {
   const HostScene& h = R.host;
   const lotus_scene_desc s = host_desc(R);
-  out.table = build_light_table(s, h.env_bound ? h.env_mean : 0.0);
+  out.table = build_light_table(s, h.boxes, h.env_bound ? h.env_mean : 0.0);
   // World bounds: each instance's geometry box through its transform.
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (uint32_t i = 0; i < s.instance_count; ++i) {
@@ -1504,12 +1544,13 @@ int32_t update_scene(Renderer& R, const lotus_scene_desc& s, lotus_scene_result&
   cudaEventRecord(R.ev_start, st);
   // The host copy: every geometry's arrays, the materials, the instances.
   HostScene& h = R.host;
+  HostArena<float> positions = std::move(h.positions);
+  HostArena<uint32_t> triangles = std::move(h.triangles);
   h = HostScene{};
+  h.positions = std::move(positions);
+  h.triangles = std::move(triangles);
   const uint32_t ng = s.geometry_count;
-  h.positions.resize(ng);
-  h.triangles.resize(ng);
-  h.normals.resize(ng);
-  h.geometries.resize(ng);
+  h.geometries.assign(s.geometries, s.geometries + ng);
   h.boxes.resize(ng);
   h.vertex_base.resize(ng);
   h.node_base.resize(ng);
@@ -1518,28 +1559,32 @@ int32_t update_scene(Renderer& R, const lotus_scene_desc& s, lotus_scene_result&
   uint64_t nodes = 0, tri_total = 0, normal_total = 0, vert_total = 0;
   for (uint32_t g = 0; g < ng; ++g) {
     const lotus_geometry& geo = s.geometries[g];
-    h.positions[g].assign(geo.positions, geo.positions + 3ull * geo.vertex_count);
-    h.triangles[g].assign(geo.triangles, geo.triangles + 3ull * geo.triangle_count);
-    if (geo.normals && geo.triangle_count) h.normals[g].assign(geo.normals, geo.normals + 9ull * geo.triangle_count);
-    lotus_geometry& copy = h.geometries[g];
-    copy = geo;
-    copy.positions = h.positions[g].data();
-    copy.triangles = h.triangles[g].data();
-    copy.normals = h.normals[g].empty() ? nullptr : h.normals[g].data();
-    copy.texcoords = nullptr;  // on the device only
-    copy.colors = nullptr;
-    copy.color_counts = nullptr;
-    h.boxes[g] = geometry_box(copy);
     h.vertex_base[g] = vert_total;
     h.node_base[g] = (uint32_t)nodes;
     h.tri_base[g] = (uint32_t)tri_total;
-    nodes += BvhBuilder::node_count(geo.triangle_count);
-    tri_total += geo.triangle_count;
-    vert_total += geo.vertex_count;
-    if (copy.normals) {
+    if (geo.normals && geo.triangle_count) {
       h.normal_base[g] = (uint32_t)normal_total;
       normal_total += geo.triangle_count;
     }
+    nodes += BvhBuilder::node_count(geo.triangle_count);
+    tri_total += geo.triangle_count;
+    vert_total += geo.vertex_count;
+  }
+  float* all_positions = h.positions.need(3 * vert_total);
+  uint32_t* all_triangles = h.triangles.need(3 * tri_total);
+  for (uint32_t g = 0; g < ng; ++g) {
+    const lotus_geometry& geo = s.geometries[g];
+    lotus_geometry& copy = h.geometries[g];
+    copy.positions = all_positions + 3 * h.vertex_base[g];
+    copy.triangles = all_triangles + 3 * (size_t)h.tri_base[g];
+    if (geo.vertex_count) std::memcpy(all_positions + 3 * h.vertex_base[g], geo.positions, 12ull * geo.vertex_count);
+    if (geo.triangle_count)
+      std::memcpy(all_triangles + 3 * (size_t)h.tri_base[g], geo.triangles, 12ull * geo.triangle_count);
+    copy.normals = nullptr;  // on the device only, as the ones below
+    copy.texcoords = nullptr;
+    copy.colors = nullptr;
+    copy.color_counts = nullptr;
+    h.boxes[g] = geometry_box(copy);
   }
   h.nodes = nodes;
   h.materials.assign(s.materials, s.materials + s.material_count);
@@ -1556,33 +1601,25 @@ int32_t update_scene(Renderer& R, const lotus_scene_desc& s, lotus_scene_result&
       !R.ok(R.tris.resize(kTriStride * std::max<uint64_t>(tri_total, 1)), "triangle pool", detail))
     return fail(detail);
   // Every geometry's positions and triangles in one upload each; they stay
-  // resident for the incremental updates' rebuilds.
-  {
-    std::vector<float> h_pos(3 * vert_total);
-    std::vector<uint32_t> h_tri(3 * tri_total);
-    for (uint32_t g = 0; g < ng; ++g) {
-      if (!h.positions[g].empty())
-        std::memcpy(&h_pos[3 * h.vertex_base[g]], h.positions[g].data(), 4 * h.positions[g].size());
-      if (!h.triangles[g].empty())
-        std::memcpy(&h_tri[3 * (size_t)h.tri_base[g]], h.triangles[g].data(), 4 * h.triangles[g].size());
-    }
-    if (!R.ok(R.scene_pos.upload(h_pos.data(), h_pos.size(), st), "positions", detail) ||
-        !R.ok(R.scene_tri.upload(h_tri.data(), h_tri.size(), st), "triangles", detail))
-      return fail(detail);
+  // resident for the incremental updates' rebuilds. The corner normals go up
+  // from the caller's arrays.
+  if (!R.ok(R.scene_pos.upload(all_positions, 3 * vert_total, st), "positions", detail) ||
+      !R.ok(R.scene_tri.upload(all_triangles, 3 * tri_total, st), "triangles", detail))
+    return fail(detail);
+  if (normal_total) {
+    if (!R.ok(R.normals.resize(9 * normal_total), "normals", detail)) return fail(detail);
+    for (uint32_t g = 0; g < ng; ++g)
+      if (h.normal_base[g] != kNoLights &&
+          !R.ok(cudaMemcpyAsync(R.normals.ptr + 9 * (size_t)h.normal_base[g], s.geometries[g].normals,
+                    36ull * s.geometries[g].triangle_count, cudaMemcpyHostToDevice, st),
+              "normals", detail))
+        return fail(detail);
+  } else {
+    R.normals.release();
   }
   std::vector<uint32_t> all(ng);
   for (uint32_t g = 0; g < ng; ++g) all[g] = g;
   if (!build_blases(R, all, true, detail)) return fail(detail);
-  // Corner normals.
-  if (normal_total) {
-    std::vector<float> h_n(9 * normal_total);
-    for (uint32_t g = 0; g < ng; ++g)
-      if (h.normal_base[g] != kNoLights)
-        std::memcpy(&h_n[9 * (size_t)h.normal_base[g]], h.normals[g].data(), 4 * h.normals[g].size());
-    if (!R.ok(R.normals.upload(h_n.data(), h_n.size(), st), "normals", detail)) return fail(detail);
-  } else {
-    R.normals.release();
-  }
   // Materials.
   std::vector<MaterialRecord> h_mat(s.material_count);
   for (uint32_t i = 0; i < s.material_count; ++i) {
@@ -1737,29 +1774,28 @@ int32_t update_geometry(Renderer& R, uint32_t geometry, const float* positions, 
   lotus_geometry& geo = h.geometries[geometry];
   if (vertex_count != geo.vertex_count) return reject("a point edit keeps the geometry's vertex count");
   if (vertex_count && !positions) return reject("the position array is missing");
-  if ((normals != nullptr) != (geo.normals != nullptr))
+  if ((normals != nullptr) != (h.normal_base[geometry] != kNoLights))
     return reject("a point edit of a geometry with corner normals gives new ones, and none otherwise");
-  for (uint64_t i = 0; i < 3ull * vertex_count; ++i)
-    if (!std::isfinite(positions[i])) return reject("the geometry has a non-finite position");
+  if (!all_finite(positions, 3ull * vertex_count)) return reject("the geometry has a non-finite position");
   auto fail = [&](const std::string& d) {
     R.failure = d;
     R.release_scene();
     return reject(d);
   };
   cudaStream_t st = R.stream;
-  std::copy(positions, positions + 3ull * vertex_count, h.positions[geometry].begin());
-  if (normals) std::copy(normals, normals + 9ull * geo.triangle_count, h.normals[geometry].begin());
+  float* kept = h.positions.data.get() + 3 * h.vertex_base[geometry];
+  if (vertex_count) std::memcpy(kept, positions, 12ull * vertex_count);
   h.boxes[geometry] = geometry_box(geo);
   InstanceState inst;
   if (!prepare_instances(R, inst, detail)) return fail(detail);
   cudaEventRecord(R.ev_start, st);
   if (vertex_count &&
-      !R.ok(cudaMemcpyAsync(R.scene_pos.ptr + 3 * h.vertex_base[geometry], h.positions[geometry].data(),
+      !R.ok(cudaMemcpyAsync(R.scene_pos.ptr + 3 * h.vertex_base[geometry], kept,
                 12ull * vertex_count, cudaMemcpyHostToDevice, st),
           "positions", detail))
     return fail(detail);
   if (normals && geo.triangle_count &&
-      !R.ok(cudaMemcpyAsync(R.normals.ptr + 9 * (size_t)h.normal_base[geometry], h.normals[geometry].data(),
+      !R.ok(cudaMemcpyAsync(R.normals.ptr + 9 * (size_t)h.normal_base[geometry], normals,
                 36ull * geo.triangle_count, cudaMemcpyHostToDevice, st),
           "normals", detail))
     return fail(detail);
@@ -2205,7 +2241,7 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   auto find_graph = [&](const Renderer::GraphKey& key) -> Renderer::CapturedGraph& {
     Renderer::CapturedGraph* slot = &R.graphs[0];
     for (Renderer::CapturedGraph& g : R.graphs) {
-      if (g.exec && g.key == key) {
+      if (g.used && g.key == key) {
         slot = &g;
         break;
       }
@@ -2215,6 +2251,7 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
       cudaGraphExecDestroy(slot->exec);
       slot->exec = nullptr;
     }
+    if (!(slot->key == key)) slot->seen = false;
     slot->key = key;
     slot->used = ++R.graph_clock;
     return *slot;
@@ -2243,7 +2280,10 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
       if (!chain.exec) {
         Queues QW = Q, QW2 = Q2;
         QW.capacity = QW2.capacity = w * pixels;
-        if (!R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
+        const bool capture = chain.seen;
+        chain.seen = true;
+        if (capture &&
+            !R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
           return poison(detail);
         for (uint32_t j = 0; j < count; ++j) launch_wave_frame(fc0, fc0 + 1 + j, w * j, w, pixels, s);
         if (count > 1) {
@@ -2262,9 +2302,9 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
           cudaStreamWaitEvent(s, R.ev_join, 0);
         }
         launch_advance_by(fc0, w * count, s);
-        if (!end_capture(chain)) return poison(detail);
+        if (capture ? !end_capture(chain) : !R.ok(cudaGetLastError(), "launch", detail)) return poison(detail);
       }
-      if (!R.ok(cudaGraphLaunch(chain.exec, s), "graph launch", detail)) return poison(detail);
+      if (chain.exec && !R.ok(cudaGraphLaunch(chain.exec, s), "graph launch", detail)) return poison(detail);
       k += w * count;
       last_counts = ((count - 1) & 1u) ? R.counts2.ptr : R.counts.ptr;
       last_wave = w;
@@ -2302,14 +2342,17 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
       gk.wave = gk.count = 0;
       Renderer::CapturedGraph& one = find_graph(gk);
       if (!one.exec) {
-        if (!R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
+        const bool capture = one.seen;
+        one.seen = true;
+        if (capture &&
+            !R.ok(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture", detail))
           return poison(detail);
         launch_wavefront_sample(R.view, R.frame_const.ptr, rect, t.width, t.height, st.max_bounces, P, Q,
             R.accum.ptr, R.color.ptr, R.totals.ptr, s, nullptr, tuning, &cq);
         launch_advance(R.frame_const.ptr, s);
-        if (!end_capture(one)) return poison(detail);
+        if (capture ? !end_capture(one) : !R.ok(cudaGetLastError(), "launch", detail)) return poison(detail);
       }
-      if (!R.ok(cudaGraphLaunch(one.exec, s), "graph launch", detail)) return poison(detail);
+      if (one.exec && !R.ok(cudaGraphLaunch(one.exec, s), "graph launch", detail)) return poison(detail);
     } else {
       launch_reference_pt(R.view, R.frame_const.ptr, rect, R.accum.ptr, R.color.ptr, R.totals.ptr, s);
       launch_advance(R.frame_const.ptr, s);
