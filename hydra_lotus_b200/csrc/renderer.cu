@@ -3069,8 +3069,9 @@ int32_t render_temporal(Renderer& R, const lotus_temporal_desc& td, lotus_frame_
     return poison(detail);
   cudaEventRecord(R.ev_start, s);
   const uint32_t pixels = (uint32_t)n;
-  launch_temporal_surface(R.view, R.frame_const.ptr, T.constants.ptr, T.instances.ptr, T.surface[sw].ptr, pixels, s);
-  launch_reproject(T.constants.ptr, T.surface[sw].ptr, T.surface[1 - sw].ptr, T.validity.ptr, pixels, s);
+  const uint32_t blocks = tile_blocks(t.width, t.height);
+  launch_temporal_surface(R.view, R.frame_const.ptr, T.constants.ptr, T.instances.ptr, T.surface[sw].ptr, blocks, s);
+  launch_reproject(T.constants.ptr, T.surface[sw].ptr, T.surface[1 - sw].ptr, T.validity.ptr, blocks, s);
   if (restir) {
     const VisibilityQueue vq{T.vis_origin.ptr, T.vis_direction.ptr, T.vis_slot.ptr, T.vis_pending.ptr,
         T.vis_counters.ptr, pixels, T.vis_counters.ptr + 2 * kVisibilityPasses};
@@ -3079,19 +3080,19 @@ int32_t render_temporal(Renderer& R, const lotus_temporal_desc& td, lotus_frame_
         !R.ok(cudaMemsetAsync(vq.failed, 0xFF, kVisibilityPasses * sizeof(uint32_t), s), "visibility queue", detail))
       return poison(detail);
     launch_restir_initial(R.view, R.frame_const.ptr, T.constants.ptr, T.initial.ptr, T.primary_hit.ptr,
-        T.primary_rng.ptr, vq, pixels, s);
+        T.primary_rng.ptr, vq, blocks, s);
     launch_visibility(R.view, vq, 0, reinterpret_cast<unsigned char*>(T.initial.ptr), sizeof(RestirPixel), false,
         s, R.tuning);
     if (reservoirs) {
       launch_restir_temporal(R.view, R.frame_const.ptr, T.constants.ptr, T.primary_hit.ptr, T.instances.ptr,
           T.initial.ptr, T.validity.ptr, T.surface[sw].ptr, T.reuse[1 - rs].ptr, T.surfaces[1 - rs].ptr,
-          T.reuse[rs].ptr, T.surfaces[rs].ptr, vq, pixels, s);
+          T.reuse[rs].ptr, T.surfaces[rs].ptr, vq, blocks, s);
       launch_visibility(R.view, vq, 1, reinterpret_cast<unsigned char*>(T.reuse[rs].ptr), sizeof(RestirReuse),
           true, s, R.tuning);
     }
     if (st.restir_spatial) {
       launch_restir_spatial(R.view, R.frame_const.ptr, T.constants.ptr, T.reuse[rs].ptr, T.surfaces[rs].ptr,
-          T.spatial.ptr, T.sources.ptr, vq, pixels, s);
+          T.spatial.ptr, T.sources.ptr, vq, blocks, s);
       launch_visibility(R.view, vq, 2, reinterpret_cast<unsigned char*>(T.spatial.ptr), sizeof(RestirReuse), true,
           s, R.tuning);
     }
@@ -3137,7 +3138,7 @@ int32_t render_temporal(Renderer& R, const lotus_temporal_desc& td, lotus_frame_
   if (accumulate) {
     cudaMemcpyAsync(T.batch.ptr, R.color.ptr, n * sizeof(float4), cudaMemcpyDeviceToDevice, s);
     launch_svgf(T.constants.ptr, tc, T.batch.ptr, T.surface[sw].ptr, T.validity.ptr, T.radiance[1 - rw].ptr,
-        T.radiance[rw].ptr, T.filter.ptr, R.color.ptr, pixels, s);
+        T.radiance[rw].ptr, T.filter.ptr, R.color.ptr, blocks, s);
   }
   cudaEventRecord(R.ev_stop, s);
   RayTotals totals{};

@@ -17,7 +17,7 @@
 namespace lotus {
 namespace {
 
-constexpr int kBlock = 128;
+constexpr int kBlock = kTileThreads;
 
 // ---------------------------------------------------------------------------
 // SVGF.
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kBlock) k_svgf_accumulate(const TemporalConst*
     RadiancePixel* __restrict__ out) {
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, tc.width, tc.height, px, py)) return;
+  if (!pixel_of(tc.width, tc.height, px, py)) return;
   const uint32_t index = py * tc.width + px;
   RadiancePixel o = {};
   o.color = batch[index];
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kBlock) k_svgf_variance(const TemporalConst* _
     float4* __restrict__ filter) {
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, tc.width, tc.height, px, py)) return;
+  if (!pixel_of(tc.width, tc.height, px, py)) return;
   const int x = (int)px, y = (int)py;
   const uint32_t index = py * tc.width + px;
   const RadiancePixel center = radiance[index];
@@ -194,7 +194,12 @@ __device__ __forceinline__ float filter_depth_step(const TemporalConst& tc, cons
   return fmaxf(step, 0.0f);
 }
 
-// FilterIteration (temporal.slang:405-457).
+// FilterIteration (temporal.slang:405-457). Bound by the latency of its 97
+// loads (7 of 16 warps a scheduler resident, an instruction in 0.55 of
+// the cycles, 44 % of L1's rate): a tap's three loads start together (1280x720,
+// five iterations: 481 us to 426), and a block's pixels form a tile (385).
+// Two to four pixels of a column to a thread, sharing their rows' taps, ran
+// slower (472 to 832 us: fewer warps), five taps loaded ahead too (434 to 543).
 __device__ __forceinline__ float4 filter_iteration(const TemporalConst& tc, const float4* __restrict__ filter,
     int x, int y, uint32_t iteration) {
   const uint32_t pixels = tc.width * tc.height;
@@ -233,19 +238,26 @@ __device__ __forceinline__ float4 filter_iteration(const TemporalConst& tc, cons
   float sx = 0.0f, sy = 0.0f, sz = 0.0f, var = 0.0f, weight_sum = 0.0f;
 #pragma unroll
   for (int ty = -2; ty <= 2; ++ty) {
+    const int qy = y + ty * step;
+    if (qy < 0 || qy >= (int)tc.height) continue;
 #pragma unroll
     for (int tx = -2; tx <= 2; ++tx) {
-      const int qx = x + tx * step, qy = y + ty * step;
-      if (!filter_neighbour(tc, filter, qx, qy, center.x, center.y, g)) continue;
-      const float4 value = in[(uint32_t)qy * tc.width + (uint32_t)qx];
+      const int qx = x + tx * step;
+      if (qx < 0 || qx >= (int)tc.width) continue;
+      // The tap's three loads start together, before its guide decides.
+      const uint32_t i = (uint32_t)qy * tc.width + (uint32_t)qx;
+      g = filter_guide(filter, pixels, i);
+      const float4 value = in[i];
+      const F3 other = V(filter[3 * (size_t)pixels + i]);
+      const float tap_lum = luminance(value.x, value.y, value.z);
+      if (g.z == kNoFilterGuide || g.x != center.x || g.y != center.y) continue;
       float w = kernel[abs(tx)] * kernel[abs(ty)];
       if (tx != 0 || ty != 0) {
-        const F3 other = V(filter[3 * (size_t)pixels + (uint32_t)qy * tc.width + (uint32_t)qx]);
         const float facing = saturate(dot(normal, other));
         // A neighbour facing away weighs 0 (pow(0, 128)): its tap adds nothing.
         if (facing == 0.0f) continue;
         const float wz = fabsf(depth - __uint_as_float(g.z)) * inv_depth[tx * tx + ty * ty];
-        const float wl = fabsf(lum - luminance(value.x, value.y, value.z)) * inv_phi_l;
+        const float wl = fabsf(lum - tap_lum) * inv_phi_l;
         const float wn = powf(facing, 128.0f);
         w = w * expf(-(wl + wz)) * wn;
       }
@@ -267,7 +279,7 @@ __global__ void __launch_bounds__(kBlock) k_svgf_filter(const TemporalConst* __r
     float4* __restrict__ color) {
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, tc.width, tc.height, px, py)) return;
+  if (!pixel_of(tc.width, tc.height, px, py)) return;
   const uint32_t index = py * tc.width + px;
   const uint32_t pixels = tc.width * tc.height;
   if (!composite) {
@@ -291,21 +303,19 @@ __global__ void k_copy_radiance_color(const TemporalConst* __restrict__ tcp,
   if (i < tc.width * tc.height) color[i] = radiance[i].color;
 }
 
-inline uint32_t grid(uint32_t n) { return (n + kBlock - 1) / kBlock; }
-
 }  // namespace
 
 void launch_svgf(const TemporalConst* tc, const TemporalConst& host_tc, const float4* batch,
     const TemporalPixel* surface, const ValidityPixel* validity, const RadiancePixel* old,
-    RadiancePixel* radiance, float4* filter, float4* color, uint32_t pixels, cudaStream_t s) {
-  k_svgf_accumulate<<<grid(pixels), kBlock, 0, s>>>(tc, batch, surface, validity, old, radiance);
-  k_svgf_variance<<<grid(pixels), kBlock, 0, s>>>(tc, surface, radiance, filter);
+    RadiancePixel* radiance, float4* filter, float4* color, uint32_t blocks, cudaStream_t s) {
+  k_svgf_accumulate<<<blocks, kBlock, 0, s>>>(tc, batch, surface, validity, old, radiance);
+  k_svgf_variance<<<blocks, kBlock, 0, s>>>(tc, surface, radiance, filter);
   if (host_tc.filter_iterations == 0) {
-    k_copy_radiance_color<<<grid(pixels), kBlock, 0, s>>>(tc, radiance, color);
+    k_copy_radiance_color<<<(host_tc.width * host_tc.height + kBlock - 1) / kBlock, kBlock, 0, s>>>(tc, radiance, color);
     return;
   }
   for (uint32_t i = 0; i < host_tc.filter_iterations; ++i)
-    k_svgf_filter<<<grid(pixels), kBlock, 0, s>>>(tc, filter, i, i + 1 == host_tc.filter_iterations ? 1u : 0u,
+    k_svgf_filter<<<blocks, kBlock, 0, s>>>(tc, filter, i, i + 1 == host_tc.filter_iterations ? 1u : 0u,
         radiance, surface, color);
 }
 

@@ -14,7 +14,7 @@
 namespace lotus {
 namespace {
 
-constexpr int kBlock = 128;
+constexpr int kBlock = kTileThreads;
 
 __device__ __forceinline__ bool in_rect(const FrameConst& f, uint32_t px, uint32_t py) {
   return px >= f.rect[0] && py >= f.rect[1] && px < f.rect[0] + f.rect[2] && py < f.rect[1] + f.rect[3];
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kBlock) k_temporal_surface(SceneView S,
   const FrameConst& f = *fcp;
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, f.width, f.height, px, py)) return;
+  if (!pixel_of(f.width, f.height, px, py)) return;
   const uint32_t index = py * f.width + px;
   TemporalPixel o = {};
   if (in_rect(f, px, py)) {
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kBlock) k_reproject(const TemporalConst* __res
     ValidityPixel* __restrict__ out) {
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, tc.width, tc.height, px, py)) return;
+  if (!pixel_of(tc.width, tc.height, px, py)) return;
   const uint32_t index = py * tc.width + px;
   const TemporalPixel cur = current[index];
   ValidityPixel o = {0u, 0u, 0xffffffffu, 0u};
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kBlock, kRestirBlocksPerSm) k_restir_initial(S
   const FrameConst& f = *fcp;
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, f.width, f.height, px, py)) return;
+  if (!pixel_of(f.width, f.height, px, py)) return;
   const uint32_t slot = py * f.width + px;
   RestirPixel r = empty_restir_pixel();
   const bool active = tc.restir_candidates != 0 && in_rect(f, px, py);
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kBlock, kRestirBlocksPerSm) k_restir_temporal(
   const FrameConst& f = *fcp;
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, f.width, f.height, px, py)) return;
+  if (!pixel_of(f.width, f.height, px, py)) return;
   const uint32_t slot = py * f.width + px;
   RestirReuse result = {};
   RestirSurface receiver = {};
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(kBlock, kRestirBlocksPerSm) k_restir_spatial(S
   const FrameConst& f = *fcp;
   const TemporalConst& tc = *tcp;
   uint32_t px, py;
-  if (!pixel_of(blockIdx.x * blockDim.x + threadIdx.x, f.width, f.height, px, py)) return;
+  if (!pixel_of(f.width, f.height, px, py)) return;
   const uint32_t slot = py * f.width + px;
   const RestirReuse centre = temporal[slot];
   const RestirSurface receiver = surfaces[slot];
@@ -623,46 +623,44 @@ __global__ void __launch_bounds__(kBlock, kRestirBlocksPerSm) k_restir_spatial(S
   out_sources[slot] = make_uint4(sources[0], sources[1], sources[2], sources[3]);
 }
 
-inline uint32_t grid(uint32_t n) { return (n + kBlock - 1) / kBlock; }
-
 }  // namespace
 
 void launch_temporal_surface(const SceneView& S, const FrameConst* fc, const TemporalConst* tc,
-    const TemporalInstance* ids, TemporalPixel* out, uint32_t pixels, cudaStream_t s) {
-  if (S.full_shading) k_temporal_surface<true><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, ids, out);
-  else k_temporal_surface<false><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, ids, out);
+    const TemporalInstance* ids, TemporalPixel* out, uint32_t blocks, cudaStream_t s) {
+  if (S.full_shading) k_temporal_surface<true><<<blocks, kBlock, 0, s>>>(S, fc, tc, ids, out);
+  else k_temporal_surface<false><<<blocks, kBlock, 0, s>>>(S, fc, tc, ids, out);
 }
 
 void launch_reproject(const TemporalConst* tc, const TemporalPixel* current, const TemporalPixel* previous,
-    ValidityPixel* out, uint32_t pixels, cudaStream_t s) {
-  k_reproject<<<grid(pixels), kBlock, 0, s>>>(tc, current, previous, out);
+    ValidityPixel* out, uint32_t blocks, cudaStream_t s) {
+  k_reproject<<<blocks, kBlock, 0, s>>>(tc, current, previous, out);
 }
 
 void launch_restir_initial(const SceneView& S, const FrameConst* fc, const TemporalConst* tc,
-    RestirPixel* out, uint4* primary_hit, uint32_t* primary_rng, const VisibilityQueue& vq, uint32_t pixels,
+    RestirPixel* out, uint4* primary_hit, uint32_t* primary_rng, const VisibilityQueue& vq, uint32_t blocks,
     cudaStream_t s) {
-  if (S.full_shading) k_restir_initial<true><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, out, primary_hit, primary_rng, vq);
-  else k_restir_initial<false><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, out, primary_hit, primary_rng, vq);
+  if (S.full_shading) k_restir_initial<true><<<blocks, kBlock, 0, s>>>(S, fc, tc, out, primary_hit, primary_rng, vq);
+  else k_restir_initial<false><<<blocks, kBlock, 0, s>>>(S, fc, tc, out, primary_hit, primary_rng, vq);
 }
 
 void launch_restir_temporal(const SceneView& S, const FrameConst* fc, const TemporalConst* tc,
     const uint4* primary_hit, const TemporalInstance* ids, const RestirPixel* initial,
     const ValidityPixel* validity, const TemporalPixel* surface, const RestirReuse* previous,
     const RestirSurface* previous_surfaces, RestirReuse* out, RestirSurface* out_surfaces,
-    const VisibilityQueue& vq, uint32_t pixels, cudaStream_t s) {
+    const VisibilityQueue& vq, uint32_t blocks, cudaStream_t s) {
   if (S.full_shading)
-    k_restir_temporal<true><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, primary_hit, ids, initial, validity, surface,
+    k_restir_temporal<true><<<blocks, kBlock, 0, s>>>(S, fc, tc, primary_hit, ids, initial, validity, surface,
         previous, previous_surfaces, out, out_surfaces, vq);
   else
-    k_restir_temporal<false><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, primary_hit, ids, initial, validity, surface,
+    k_restir_temporal<false><<<blocks, kBlock, 0, s>>>(S, fc, tc, primary_hit, ids, initial, validity, surface,
         previous, previous_surfaces, out, out_surfaces, vq);
 }
 
 void launch_restir_spatial(const SceneView& S, const FrameConst* fc, const TemporalConst* tc,
     const RestirReuse* temporal, const RestirSurface* surfaces, RestirReuse* out, uint4* sources,
-    const VisibilityQueue& vq, uint32_t pixels, cudaStream_t s) {
-  if (S.full_shading) k_restir_spatial<true><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, temporal, surfaces, out, sources, vq);
-  else k_restir_spatial<false><<<grid(pixels), kBlock, 0, s>>>(S, fc, tc, temporal, surfaces, out, sources, vq);
+    const VisibilityQueue& vq, uint32_t blocks, cudaStream_t s) {
+  if (S.full_shading) k_restir_spatial<true><<<blocks, kBlock, 0, s>>>(S, fc, tc, temporal, surfaces, out, sources, vq);
+  else k_restir_spatial<false><<<blocks, kBlock, 0, s>>>(S, fc, tc, temporal, surfaces, out, sources, vq);
 }
 
 }  // namespace lotus
