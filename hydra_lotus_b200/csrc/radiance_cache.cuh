@@ -12,6 +12,8 @@
 
 #include <cuda_fp16.h>
 
+#include <mutex>
+
 #include "common.cuh"
 
 namespace lotus {
@@ -112,7 +114,19 @@ class RadianceCache {
  private:
   cudaError_t pack(cudaStream_t s);
   cudaError_t adam_kernels(cudaStream_t s);
+  cudaError_t workspace(int k, size_t bytes, void** out);
 
+  struct HostCall {
+    explicit HostCall(RadianceCache& c) : cache(c), lock(c.host_calls_) {}
+    ~HostCall();
+    RadianceCache& cache;
+    std::lock_guard<std::mutex> lock;
+  };
+  static constexpr int kWorkspaces = 3;
+  static constexpr size_t kKeptWorkspace = size_t(64) << 20;
+  void* workspace_[kWorkspaces] = {};
+  size_t workspace_bytes_[kWorkspaces] = {};
+  std::mutex host_calls_;
   CacheConfig config_;
   CacheGrid grid_{};
   float* master_ = nullptr;     // FP32 weights

@@ -3,6 +3,8 @@ the tensor-core forward and backward passes against the FP64 oracle
 (oracle/cache_oracle.py) on the same BF16-rounded operands, the query
 encoding, and training with Adam on a known function."""
 
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -196,3 +198,22 @@ def test_cache_timings_split(cuda):
     assert res.cache_queries > 0 and res.cache_training_records > 0
     assert res.cache_infer_gpu_ms > 0.0 and res.cache_train_gpu_ms > 0.0
     assert abs(res.cache_infer_gpu_ms + res.cache_train_gpu_ms - res.cache_gpu_ms) < 1e-9
+
+
+def test_workspaces(cuda):
+    """Calls of growing and shrinking sizes, below and above the bytes a
+    cache keeps (64 MiB), and calls from several threads at once, each give
+    what their own records give alone."""
+    rng = np.random.default_rng(11)
+    scene = scenes.box_room(seed=0, size=32)
+    with cuda.CudaOffscreenRenderer(0) as r:
+        cuda.check(r.update_scene(scene), "update_scene")
+        r.configure_cache(enable=False, seed=7)
+        big = rng.uniform(-1.0, 1.0, size=((64 << 20) // 256 + 77, 64)).astype(np.float32)
+        want = r.cache_infer(big)
+        for start, n in ((0, 1), (5, 128), (0, len(big)), (1000, 129), (3, 40000), (0, len(big))):
+            assert np.array_equal(r.cache_infer(big[start:start + n]), want[start:start + n])
+        with ThreadPoolExecutor(4) as pool:
+            spans = [(k * 997, 300 + 131 * k) for k in range(16)]
+            for (start, n), got in zip(spans, pool.map(lambda a: r.cache_infer(big[a[0]:a[0] + a[1]]), spans)):
+                assert np.array_equal(got, want[start:start + n])
