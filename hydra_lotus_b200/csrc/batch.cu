@@ -365,7 +365,7 @@ extern "C" int32_t lotus_cuda_batch_render(lotus_cuda_batch* b, const lotus_fram
   bool analytic = false, full_shading = false;
   // Every scene's walks report to the first scene's walk-failure words.
   uint32_t* walk_failure = nullptr;
-  uint32_t step_limit = kMaxTraversalSteps;
+  uint32_t step_limit = 0xFFFFFFFFu;  // the smallest of the scenes'
   for (uint32_t k = 0; k < count; ++k) {
     RendererAccess a;
     if (!renderer_access(b->scenes[k], a, detail)) return fail("scene " + std::to_string(k) + ": " + detail);

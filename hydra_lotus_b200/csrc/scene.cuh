@@ -662,8 +662,9 @@ __device__ __forceinline__ void walk_pop(Walk& W, const WalkStack& stack, uint32
 
 // A walk that has ended: if it ended on its step budget or a stack
 // overflow, its hits may be incomplete; count it and record the cause.
-__device__ __forceinline__ void walk_check_end(const SceneView& S, const Walk& W) {
-  if (W.steps >= S.step_limit) {
+// `limit` is the budget that the walk was held to.
+__device__ __forceinline__ void walk_check_end(const SceneView& S, const Walk& W, uint32_t limit) {
+  if (W.steps >= limit) {
     atomicAdd(&S.walk_failure[0], 1u);
     atomicOr(&S.walk_failure[1], (W.steps & kWalkOverflow) ? kWalkFailedStack : kWalkFailedSteps);
   }
@@ -812,7 +813,7 @@ __device__ __forceinline__ float traverse(const SceneView& S, F3 origin, F3 dire
       break;
     }
   }
-  walk_check_end(S, W);
+  walk_check_end(S, W, limit);
   found = W.is(kWalkFound);
   if (!kAnyHit && found) hit = Hit{store.hit_instance, store.hit_tri, store.hit_b1, store.hit_b2, W.best};
   return kAnyHit ? W.transmittance : 0.0f;
@@ -858,7 +859,7 @@ __device__ __forceinline__ bool walk_round(const SceneView& S, Walk& W, Store& s
   if (active && !ended && W.cur != kWalkDone && !walk_at_node(W))
     ended = walk_other<kAnyHit, kCount, kFullShading>(S, W, store, stack, rng, limit, counters);
   const bool done = active && (ended || (W.cur == kWalkDone && W.leaf == 0));
-  if (done) walk_check_end(S, W);
+  if (done) walk_check_end(S, W, limit);
   return done;
 }
 
