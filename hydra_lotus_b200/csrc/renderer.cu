@@ -655,7 +655,7 @@ constexpr uint32_t kMaxChain = 4;
 // small target leave most of a launch to its ramp-up and drain and the tail
 // kernel most of the frame, a wave holds up to kMaxSmallWave samples of at
 // most kWavePaths paths together (2^21 paths: 344 MB of path state and
-// queues). Box room at 256 squared, 64 samples: 5.36 ms in eights, 5.07 with
+// queues, and as much again for the second wave in flight). Box room at 256 squared, 64 samples: 5.36 ms in eights, 5.07 with
 // waves of 2^20 paths, 4.59 with 2^21, 4.60 with 2^22; the texture fixture
 // at 161 squared, 128 samples: 4.58, 3.67, 3.08 and 3.09 ms (its tail kernel
 // 2.53 -> 0.25).
@@ -1835,13 +1835,32 @@ int32_t update_geometry(Renderer& R, uint32_t geometry, const float* positions, 
   return LOTUS_PASS;
 }
 
+// Both path state and queue sets, given back.
+void release_path_state(Renderer& R) {
+  R.path_origin.release(); R.path_direction.release(); R.path_throughput.release();
+  R.path_radiance.release(); R.path_hit.release();
+  R.queue_ray0.release(); R.queue_ray1.release(); R.queue_hit.release();
+  R.sq_o.release(); R.sq_d.release(); R.sq_fl.release(); R.sq_thr.release();
+  R.sort_keys.release(); R.sort_queue.release();
+  R.path_origin2.release(); R.path_direction2.release(); R.path_throughput2.release();
+  R.path_radiance2.release(); R.path_hit2.release();
+  R.queue_ray02.release(); R.queue_ray12.release(); R.queue_hit2.release();
+  R.sq_o2.release(); R.sq_d2.release(); R.sq_fl2.release(); R.sq_thr2.release();
+  R.sort_keys2.release(); R.sort_queue2.release();
+}
+
 // The targets and, for the queue kernels, a path state and queues of at
-// least `slots` paths, which a larger target or wave grows and the others
-// keep.
+// least `slots` paths, which a larger target or wave grows. Another target
+// keeps the arrays (small targets in turn do not allocate again), unless
+// they hold more than kWavePaths paths and twice what its call needs: at 164
+// bytes a path, a 3840x2160 call's two sets are 21.8 GB, which a preview
+// after it would otherwise hold on to.
 bool ensure_targets(Renderer& R, uint32_t w, uint32_t h, size_t slots, std::string& detail) {
   const size_t n = (size_t)w * h;
   bool moved = false;
   if (R.width != w || R.height != h) {
+    const size_t most = std::max((size_t)kWavePaths, 2 * slots);
+    if (R.path_origin.count > most || R.path_origin2.count > most) release_path_state(R);
     R.accum.release();
     R.color.release();
     R.depth.release();

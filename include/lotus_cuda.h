@@ -462,9 +462,12 @@ typedef struct lotus_cuda_options {
   /* Samples a RenderScene call that adds several runs in one wavefront
    * (their paths side by side in one set of queues, so that each launch
    * pays its ramp-up and drain once for all of them): 1, 2, 4 or 8; 0: 8,
-   * and on small targets as many as keep 2^21 paths in a wave, up to 64. The
-   * path state and queues take this many times the target's pixels. Results
-   * do not depend on it. */
+   * and on small targets as many as keep 2^21 paths in a wave, up to 64.
+   * Two waves are in flight at a time, each with path state and queues of
+   * 164 bytes a path: two sets of this many times the target's pixels. A
+   * renderer keeps the largest sets its calls have needed; a call on a target
+   * of another size gives them back first where they hold more than 2^21
+   * paths and twice what that call needs. Results do not depend on it. */
   uint32_t samples_per_wave;
 } lotus_cuda_options;
 
