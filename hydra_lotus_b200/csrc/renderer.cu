@@ -2000,12 +2000,12 @@ using namespace lotus;
 
 // The samples a call that adds `samples` runs in one wave: the options', or
 // kDefaultWave, doubled while kWavePaths and kMaxSmallWave allow it and two
-// such waves still fit into the call (two are in flight at a time); halved
-// while the call adds fewer.
-uint32_t call_wave(const Renderer& R, uint32_t pixels, uint32_t samples) {
+// such waves still fit into the call (two are in flight at a time), up to
+// `most`; halved while the call adds fewer.
+uint32_t call_wave(const Renderer& R, uint32_t pixels, uint32_t samples, uint32_t most = kMaxSmallWave) {
   uint32_t wave = R.wave ? R.wave : kDefaultWave;
   if (R.wave == 0)
-    while (wave < kMaxSmallWave && 2ull * wave * pixels <= kWavePaths && 4ull * wave <= samples) wave *= 2;
+    while (wave < most && 2ull * wave * pixels <= kWavePaths && 4ull * wave <= samples) wave *= 2;
   while (wave > 1 && wave > samples) wave /= 2;
   return wave;
 }
@@ -2058,17 +2058,35 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   // frame is latency-bound and the per-thread loop (k_reference_pt) is
   // faster. The frame's evidence stays the reference integrator's.
   const uint32_t pixels = t.width * t.height;
-  const uint64_t launch_paths = (uint64_t)pixels * call_wave(R, pixels, d.frame_count);
-  const bool queued = wavefront ||
-      (st.integrator == LOTUS_INTEGRATOR_REFERENCE && st.light_sampling <= LOTUS_LIGHT_SAMPLING_MIS &&
-       st.output == LOTUS_OUTPUT_RADIANCE && launch_paths >= extension_resident_threads());
+  const uint32_t profiled_flags = LOTUS_FRAME_TIMINGS | LOTUS_FRAME_COUNT_VISITS;
   // The radiance cache serves the wavefront integrator's samples.
   const bool use_cache = wavefront && R.cache_enabled && R.cache.ready();
-  // Path state for the call's waves at once: made for one sample and grown
-  // below, a new target's first call paid for both (1280x720: 44 ms, 14 of
-  // them the second set and freeing the first; now 35).
-  const size_t slots = !queued ? 0 : use_cache ? pixels : (size_t)launch_paths;
-  if (!ensure_targets(R, t.width, t.height, slots, detail)) return poison(detail);
+  bool queued = false;
+  uint32_t most_wave = kMaxSmallWave;
+  for (;;) {
+    const uint32_t wave = call_wave(R, pixels, d.frame_count, most_wave);
+    const uint64_t launch_paths = (uint64_t)pixels * wave;
+    queued = wavefront ||
+        (st.integrator == LOTUS_INTEGRATOR_REFERENCE && st.light_sampling <= LOTUS_LIGHT_SAMPLING_MIS &&
+         st.output == LOTUS_OUTPUT_RADIANCE && launch_paths >= extension_resident_threads());
+    // Path state for the call's waves at once: made for one sample and grown
+    // below, a new target's first call paid for both (1280x720: 44 ms, 14 of
+    // them the second set and freeing the first; now 35).
+    const size_t slots = !queued ? 0 : use_cache ? pixels : (size_t)launch_paths;
+    // A wave of more than kDefaultWave samples takes up to four or eight
+    // times that wave's memory: where the device has not got it (for both
+    // waves in flight), the call runs waves of kDefaultWave.
+    const bool large = slots > (size_t)kDefaultWave * pixels;
+    const uint32_t chained = d.frame_count - ((d.flags & profiled_flags) ? wave : 0u);
+    if (ensure_targets(R, t.width, t.height, slots, detail) &&
+        (!large || chained < 2 * wave || ensure_pair_buffers(R, slots, detail)))
+      break;
+    if (!large) return poison(detail);
+    cudaGetLastError();
+    release_path_state(R);
+    ++R.buffer_generation;
+    most_wave = kDefaultWave;
+  }
   if (use_cache && !ensure_cache_queues(R, t.width * t.height, detail)) return poison(detail);
   const CacheQueues cq = use_cache ? cache_queues(R) : CacheQueues();
   // DisplayViewport and DataScissor (vulkan_backend.cpp:651-677).
@@ -2241,7 +2259,7 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   // stream j % 2, each resolving (its samples in order) after wave j - 1, so
   // that only the chain's last tail runs alone. A call's profiled part
   // (timings or visit counts) is its last wave (or sample), run alone.
-  const uint32_t wave = call_wave(R, pixels, to_add);
+  const uint32_t wave = call_wave(R, pixels, to_add, most_wave);
   const bool waves = queued && !use_cache && to_add >= 2 && wave >= 2;
   const uint32_t profiled_samples = (want_timings || want_visits) ? (waves ? wave : 1u) : 0u;
   const uint32_t chainable = waves ? submissions - profiled_samples : 0u;

@@ -56,3 +56,29 @@ def test_small_targets_in_turn_keep_their_arrays(cuda):
         render(cuda, r, other, 1)
         assert abs(free_bytes() - before) < (64 << 20)
         assert np.array_equal(render(cuda, r, small, 64), image)
+
+
+def test_large_waves_need_not_fit(cuda):
+    """Where the device has no memory for two waves of 2^21 paths, a call that
+    waves of eight samples fit runs in those, to the same image."""
+    import torch
+
+    scene = scenes.box_room(seed=0, size=256)
+    with cuda.CudaOffscreenRenderer(0) as r:
+        cuda.check(r.update_scene(scene), "update_scene")
+        want = render(cuda, r, scene, 64)
+    large, default = 2 * WAVE_PATHS * BYTES_PER_PATH, 2 * 8 * scene.width * scene.height * BYTES_PER_PATH
+    left = (large + default) // 2  # 430 MB
+    filler = None
+    with cuda.CudaOffscreenRenderer(0) as r:
+        cuda.check(r.update_scene(scene), "update_scene")
+        try:
+            filler = torch.empty(free_bytes() - left, dtype=torch.uint8, device="cuda:0")
+            assert default < free_bytes() < large
+            images = [render(cuda, r, scene, 64), render(cuda, r, scene, 64, first=64), render(cuda, r, scene, 64)]
+        finally:
+            del filler
+            torch.cuda.empty_cache()
+        images.append(render(cuda, r, scene, 64, first=128))
+        images.append(render(cuda, r, scene, 64))
+    assert np.array_equal(images[0], want) and np.array_equal(images[2], want) and np.array_equal(images[4], want)
