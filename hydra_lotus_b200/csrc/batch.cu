@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/lotus_cuda.h"
+#include "host_pages.h"
 #include "integrator.cuh"
 #include "renderer_internal.cuh"
 
@@ -482,6 +483,11 @@ extern "C" int32_t lotus_cuda_batch_render(lotus_cuda_batch* b, const lotus_fram
     i += last_pair ? 2 : 1;
   }
   cudaEventRecord(b->ev_stop, s);
+  // The caller's image pages are mapped while the device renders, before the
+  // first copy into host memory waits for it.
+  for (uint32_t k = 0; colors && k < count; ++k)
+    if (colors[k] && frames[k].target.read_back)
+      populate_pages(colors[k], sizeof(float4) * (base[k + 1] - base[k]));
   RayTotals totals{};
   cudaMemcpyAsync(&totals, b->totals, sizeof(totals), cudaMemcpyDeviceToHost, s);
   uint32_t walks[2] = {0, 0};
