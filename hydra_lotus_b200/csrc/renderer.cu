@@ -663,24 +663,29 @@ constexpr uint32_t kDefaultWave = 8;
 constexpr uint32_t kMaxSmallWave = 64;
 constexpr uint64_t kWavePaths = 1ull << 21;
 
-// The resident scene as the incremental updates need it: each geometry's
-// arrays (owned copies; `geometries` points into them), its box and its
-// places in the device arrays and pools, the materials and the
-// environment's summary.
+// Host memory that a later, similar scene uses again.
 template <typename T>
 struct HostArena {
   std::unique_ptr<T[]> data;
   size_t capacity = 0;
-  // Uninitialised room for n elements; what it held is lost when it grows.
+  // Uninitialised room for n elements; what it held is lost when it moves.
+  // More than kKeptBytes are given back where n needs less than a quarter.
   T* need(size_t n) {
-    if (n > capacity) {
+    if (n > capacity || (capacity * sizeof(T) > kKeptBytes && n < capacity / 4)) {
+      data.reset();
+      capacity = 0;
       data.reset(new T[n]);
       capacity = n;
     }
     return data.get();
   }
+  static constexpr size_t kKeptBytes = size_t(16) << 20;
 };
 
+// The resident scene as the incremental updates need it: each geometry's
+// positions and triangles (owned copies; `geometries` points into them; the
+// corner normals are on the device only), its box and its places in the
+// device arrays and pools, the materials and the environment's summary.
 struct HostScene {
   // Every geometry's positions and triangles, one after another (at its
   // vertex_base and tri_base), as the device arrays hold them: one copy from
