@@ -15,6 +15,10 @@ from . import build_ref
 _lib = None
 
 
+class NotBuilt(RuntimeError):
+    """The reference's CPU code is not there and cannot be built here."""
+
+
 def available():
     return build_ref.build() is not None and os.path.exists(build_ref.LIB)
 
@@ -24,7 +28,7 @@ def lib():
     if _lib is None:
         path = build_ref.build()
         if path is None or not os.path.exists(path):
-            raise RuntimeError("oracle/_ref/libref.so is not built (needs the reference tree once)")
+            raise NotBuilt("oracle/_ref/libref.so is not built (needs the reference tree once)")
         L = C.CDLL(path)
         vp = C.c_void_p
         L.ref_estimate_variance.restype = C.c_float
