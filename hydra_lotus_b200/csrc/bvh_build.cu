@@ -27,7 +27,6 @@ __device__ __forceinline__ float unordered(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-// Triangle boxes in object space from the geometry's positions.
 // Folds a warp's primitive centroids into the centroid bounds with one
 // atomic per bound (lanes without a primitive add the identities); every
 // lane of the warp takes part.
@@ -45,6 +44,7 @@ __device__ __forceinline__ void warp_centroid_bounds(uint32_t* bounds, bool vali
   }
 }
 
+// Triangle boxes in object space from the geometry's positions.
 __global__ void k_triangle_boxes(const float* __restrict__ positions,
     const uint32_t* __restrict__ triangles, uint32_t n, float4* __restrict__ lo,
     float4* __restrict__ hi, uint32_t* __restrict__ centroid_bounds) {
@@ -67,7 +67,9 @@ __global__ void k_triangle_boxes(const float* __restrict__ positions,
 }
 
 // Instance world boxes: the BLAS root box's corners through
-// world_from_object, widened by a relative margin.
+// world_from_object, widened by a relative margin. The linear BVH's build
+// also takes the centroids' bounds (`centroid_bounds`), the SAH builder the
+// instances' indices (`idx`); the other is null.
 __global__ void k_instance_boxes(const InstanceShading* __restrict__ shade,
     const InstanceTraversal* __restrict__ trav, const BvhNode* __restrict__ blas, uint32_t n,
     float4* __restrict__ lo, float4* __restrict__ hi, uint32_t* __restrict__ centroid_bounds,
@@ -103,6 +105,7 @@ __global__ void k_instance_boxes(const InstanceShading* __restrict__ shade,
   }
   lo[i] = make_float4(l[0], l[1], l[2], 0.0f);
   hi[i] = make_float4(h[0], h[1], h[2], 0.0f);
+  if (centroid_bounds == nullptr) return;
   for (int a = 0; a < 3; ++a) {
     const float c = 0.5f * (l[a] + h[a]);
     atomicMin(&centroid_bounds[a], ordered(c));
@@ -1258,8 +1261,7 @@ cudaError_t BvhBuilder::build_instances_sah(const InstanceShading* shade, const 
   const std::vector<SahJob> jobs(1, SahJob{0, n, 0, 0, 1, 1, 0, 0});
   cudaError_t e = reserve(n, stream);
   if (e != cudaSuccess || (e = upload_jobs(jobs, stream)) != cudaSuccess) return e;
-  init_bounds(bounds_, stream);
-  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, bounds_, values_);
+  k_instance_boxes<<<blocks(n), kBuildBlock, 0, stream>>>(shade, trav, blas, n, plo_, phi_, nullptr, values_);
   if ((e = sah_build(jobs, n, nodes, stream)) != cudaSuccess) return e;
   return sah_errors(stream);
 }
