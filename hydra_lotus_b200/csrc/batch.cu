@@ -59,8 +59,8 @@ struct lotus_cuda_batch {
   std::vector<uint32_t> graph_layout;
   uint32_t graph_bounces = 0;
   uint32_t graph_rounds = 0;
-  // The wavefront rounds before the tail, chosen from the first sample of a
-  // layout (choose_wavefront_rounds over every scene's pixels).
+  // The wavefront rounds before the tail, chosen from the last sample of a
+  // layout's first call (choose_wavefront_rounds over every scene's pixels).
   std::vector<uint32_t> rounds_layout;
   uint32_t rounds_bounces = 0;
   uint32_t auto_rounds = 0;

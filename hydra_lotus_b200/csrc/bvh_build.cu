@@ -1,11 +1,12 @@
 // SPDX-License-Identifier: Apache-2.0
 // On-device BVH construction, replacing the driver's BLAS/TLAS builds. Two
 // builders: a SAH builder of many BVHs at once (all of a scene's BLASes in
-// three launches, and the TLAS), and, for larger meshes, a linear BVH (Karras, "Maximizing Parallelism in the
-// Construction of BVHs, Octrees, and k-d Trees", HPG 2012) over 63-bit
-// Morton codes of the primitives' centroids, sorted by CUB's radix sort,
-// with bounds fitted bottom-up. The reference's builds are (backend/vulkan/gpu_scene.cpp:1899-1950, 2240-2322 in
-// hydra-lotus).
+// three launches, and the TLAS), and, for larger meshes, a linear BVH
+// (Karras, "Maximizing Parallelism in the Construction of BVHs, Octrees, and
+// k-d Trees", HPG 2012) over 63-bit Morton codes of the primitives'
+// centroids, sorted by CUB's radix sort, with bounds fitted bottom-up. The
+// reference's builds are (backend/vulkan/gpu_scene.cpp:1899-1950, 2240-2322
+// in hydra-lotus).
 #include "bvh_build.cuh"
 
 #include <algorithm>

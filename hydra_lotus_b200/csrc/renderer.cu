@@ -891,9 +891,10 @@ struct Renderer {
   uint64_t graph_clock = 0;
   uint32_t buffer_generation = 0;  // bumped when a target, path state or queue array moves
   // Rounds before the tail are chosen (choose_wavefront_rounds) from the
-  // queue counts of the first wave rendered with `rounds_key` (its rounds,
-  // wave, count and buffers 0), which held `rounds_samples` samples; for the
-  // temporal frames from their first sample's.
+  // queue counts of the last wave or sample of the first call rendered with
+  // `rounds_key` (its rounds, wave, count and buffers 0), which held
+  // `rounds_samples` samples; for the temporal frames from their first
+  // frame's.
   GraphKey rounds_key{}, temporal_rounds_key{};
   std::vector<uint32_t> rounds_counts;
   uint32_t rounds_samples = 0, temporal_auto_rounds = 0;
@@ -1345,9 +1346,10 @@ bool submit_instances(Renderer& R, InstanceState& in, std::string& detail) {
 }
 
 // Builds the BLASes of the geometries in `which` from the device position
-// and triangle arrays: binned SAH for those up to kSahMaxTriangles (one
-// launch), LBVH for larger ones; then collapses their node ranges (or, with
-// `whole_pool`, the whole pool at once) into the 4-wide pool.
+// and triangle arrays: SAH for those up to kSahMaxTriangles (all of them
+// together, in the SAH builder's three kernels), LBVH for larger ones; then
+// collapses their node ranges (or, with `whole_pool`, the whole pool at once)
+// into the 4-wide pool.
 bool build_blases(Renderer& R, const std::vector<uint32_t>& which, bool whole_pool, std::string& detail) {
   cudaStream_t st = R.stream;
   const HostScene& h = R.host;
@@ -2242,7 +2244,8 @@ int32_t render(Renderer& R, const lotus_frame_desc& d, lotus_frame_result& res, 
   gk.cache = use_cache ? R.cache_generation : 0u;
   const Renderer::GraphKey shape_key = gk;
   // The tuning of a wave of `samples` samples: its rounds as chosen from the
-  // first wave's queue counts, scaled to its size.
+  // queue counts of the shape's first call (its last wave's or sample's),
+  // scaled to its size.
   const bool rounds_known = R.tuning.rounds == 0 && R.rounds_samples != 0 && R.rounds_key == shape_key;
   const bool choose_rounds = queued && R.tuning.rounds == 0 && !rounds_known;
   auto wave_tuning = [&](uint32_t samples) {

@@ -447,11 +447,12 @@ typedef struct lotus_cuda_options {
   uint32_t trace_blocks_per_sm;
   /* Bounces the wavefront integrator runs as rounds before its tail kernel
    * takes the paths still queued (1..LOTUS_MAX_BOUNCES + 1). 0: RenderScene
-   * chooses them from its first sample of each scene and frame shape (run
+   * chooses them from its first call of each scene and frame shape (run
    * with LOTUS_WAVEFRONT_ROUNDS): the first bounce whose queue held fewer
-   * paths than the extension kernel keeps resident on the device at once
-   * (at least 65536); other calls use LOTUS_WAVEFRONT_ROUNDS. Results do not
-   * depend on it. */
+   * paths in that call's last wave, scaled to the samples of a later one,
+   * than the extension kernel keeps resident on the device at once (at least
+   * 65536); other calls use LOTUS_WAVEFRONT_ROUNDS. Results do not depend on
+   * it. */
   uint32_t wavefront_rounds;
   /* A BVH walk's step budget (node visits, leaf tests and instance entries);
    * 0: 2^18, which only a corrupt BVH could need. A walk that runs out of it,
