@@ -59,10 +59,10 @@ EXTEND_STATE_BYTES = 72
 NODE_BYTES, TRIANGLE_BYTES, INSTANCE_BYTES = 112, 48, 64
 # DRAM bytes (read + write) per extension ray of k_wf_extend, from an Nsight
 # Compute capture of one launch (the sphere field at 960x540, one wave of
-# eight samples, bounce 1: 2,832,833 rays in key order, 499.4 MB read +
-# 63.3 MB written, caches flushed before the launch). Scaled by rays to the
+# eight samples, bounce 1: 2,832,833 rays in key order, 474.2 MB read +
+# 60.3 MB written, caches flushed before the launch). Scaled by rays to the
 # bench's launches.
-EXTEND_DRAM_BYTES_PER_RAY = 198.6
+EXTEND_DRAM_BYTES_PER_RAY = 188.7
 # B200's nominal HBM3e bandwidth (GB/s), for the fraction against it.
 NOMINAL_HBM_GBS = 8000.0
 

@@ -497,17 +497,18 @@ constexpr float kFarMargin = 1.0f + 3.8146973e-6f;
 // r ^ (i & 7) of its 128 bytes. A warp's lanes stand at different nodes and
 // load the same row of each; at one place in every 128-byte line all of them
 // would meet in the same four shared banks, one lane a cycle (7.2 data
-// cycles a load). Rotated, the L1 data pipe went from 68% to 53% busy in the
-// extension kernel and 66% to 55% in the shadow kernel (0.886 -> 0.830 ms
-// for 2.1M shadow rays of the sphere field at 960x540).
+// cycles a load). With the rows in place and the scalar arithmetic the L1
+// data pipe was 65% busy in the extension kernel and 64% in the shadow
+// kernel, rotated and packed (slab_axis) it is 55% and 53% busy (0.900 ->
+// 0.831 ms for 2.1M shadow rays of the sphere field at 960x540).
 __host__ __device__ __forceinline__ uint32_t node_row(uint32_t index, uint32_t row) { return (row ^ index) & 7u; }
 
 // One axis: the entry and exit distances of the four children. The rows are
 // chosen by the ray's direction, the entry planes being the low ones where
 // it goes up the axis, which saves the two minima and maxima an axis and
 // child; the subtractions and products go two children at a time. With the
-// three-operand minima an interior visit takes 11% fewer instructions over
-// the whole extension kernel (1,180M -> 1,054M for 2.83M rays).
+// three-operand minima the whole extension kernel takes 9% fewer
+// instructions (1,180M -> 1,073M for 2.83M rays), in 1.66 -> 1.48 ms.
 __device__ __forceinline__ void slab_axis(const char* node, uint32_t turn, float o, float inv, float tn[4],
     float tf[4]) {
   const uint32_t off = turn ^ (inv < 0.0f ? 16u : 0u);

@@ -195,8 +195,8 @@ __device__ __forceinline__ float filter_depth_step(const TemporalConst& tc, cons
 }
 
 // FilterIteration (temporal.slang:405-457). Bound by the latency of its 97
-// loads (7 of 16 warps a scheduler resident, an instruction in 0.55 of
-// the cycles, 44 % of L1's rate): a tap's three loads start together (1280x720,
+// loads (8 of 16 warps a scheduler resident, an instruction in 0.61 of
+// the cycles, 42 % of L1's rate): a tap's three loads start together (1280x720,
 // five iterations: 481 us to 426), and a block's pixels form a tile (385).
 // Two to four pixels of a column to a thread, sharing their rows' taps, ran
 // slower (472 to 832 us: fewer warps), five taps loaded ahead too (434 to 543).
